@@ -39,7 +39,7 @@ __device__ __forceinline__ bool wait_bar_cluster(uint32_t bar, uint32_t parity, 
 // calling threads (x = 0..127) read the rows from global memory, not from the ring: shared-memory loads crawl
 // while the tensor core and the copy engine keep the banks busy, and a stage held for them stalls a ring that
 // is only four deep; the copy engine has just brought the same rows into L2.
-__device__ __forceinline__ bool colsum_global_tile(const GemmOp *op, const Tile &tc, int m_tile, int x, int lane,
+__device__ __forceinline__ bool colsum_global_tile(const GemmScalars *op, const Tile &tc, int m_tile, int x, int lane,
                                                    Ctrl *ctrl, const LaunchParams &p) {
   if (op->wait_ctr[0] >= 0) {  // step kernel: the operand's producers are done before it is read
     unsigned seen = 0u;
@@ -81,9 +81,9 @@ __device__ __forceinline__ bool colsum_global_tile(const GemmOp *op, const Tile 
 // c_first, c_first + n_epi, ... of its TMEM lane quarter, hands the accumulator back (`arrive` arrivals: a
 // warp that works without its helper twin arrives for both) and publishes the tile on the dependency
 // counters (`pub` arrivals). PAIR: a CTA of a cluster of two, draining its own 128 rows (tile row `m_tile`) of a
-// 256-row tile; the accumulator barriers are the leader's.
+// 256-row tile; the accumulator barriers are the leader's. `maps`: the op's tensor maps, which stay where the launch put them.
 template <bool PAIR>
-__device__ __forceinline__ bool epilogue_tile(const GemmOp *op, const Tile &tc, int m_tile, uint32_t tcount, bool helper,
+__device__ __forceinline__ bool epilogue_tile(const GemmScalars *op, const GemmOp *maps, const Tile &tc, int m_tile, uint32_t tcount, bool helper,
                                               int n_epi, int c_first, unsigned arrive, unsigned pub, uint32_t sbuf,
                                               uint32_t sbuf_alt, uint32_t tmem_base, Ctrl *ctrl, const LaunchParams &p, int warp, int lane) {
   const int q = warp & 3;  // TMEM lane quarter this warp may read
@@ -186,7 +186,7 @@ __device__ __forceinline__ bool epilogue_tile(const GemmOp *op, const Tile &tc, 
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            const CUtensorMap *map = pass == 0 ? &op->tmC : &op->tmC2;
+            const CUtensorMap *map = pass == 0 ? &maps->tmC : &maps->tmC2;
             if (op->atomic_out) tma_reduce_add_2d(map, bx, nb, row0);
             else tma_store_2d(map, bx, nb, row0);
             bulk_commit();

@@ -35,17 +35,12 @@ struct Tile {
   int skip;    // nothing to compute: above the causal diagonal, or an empty reduction range
 };
 
-// Advances `cursor` to the op that owns global tile `t` and decodes the tile.
 // Order inside an op: splits outermost (tiles that run together share a k-range); inside a
 // split the output tiles are walked in bands of `band_m` tile rows, row index fastest inside a
 // band. The ~148 tiles in flight then cover band_m rows x a few columns of tiles: the A rows of
 // the band stay in L2 for the whole sweep and every B column block is fetched from HBM once
 // per band instead of once per tile row.
-__device__ __forceinline__ const GemmOp *decode_tile(const GemmOp *ops, int n_ops, int t, int &cursor,
-                                                     Tile &tc) {
-  while (cursor + 1 < n_ops && t >= ops[cursor].tile_base + ops[cursor].n_tiles) ++cursor;
-  const GemmOp *op = ops + cursor;
-  int local = t - op->tile_base;
+__device__ __forceinline__ void decode_in_op(const GemmScalars *op, int local, Tile &tc) {
   tc.bh = 0;
   tc.bb = 0;
   if (op->op_kind != OPK_GEMM) {  // row-local op or attention: tiles are numbered linearly
@@ -54,7 +49,7 @@ __device__ __forceinline__ const GemmOp *decode_tile(const GemmOp *ops, int n_op
     tc.split = 0;
     tc.kb0 = tc.kb1 = 0;
     tc.skip = 0;
-    return op;
+    return;
   }
   if (op->batch > 1) {
     const int bi = local / op->tiles_per_batch;
@@ -80,7 +75,24 @@ __device__ __forceinline__ const GemmOp *decode_tile(const GemmOp *ops, int n_op
     }
     if (tc.kb0 >= tc.kb1) tc.skip = 1;
   }
+}
+
+// Advances `cursor` to the op that owns global tile `t` and decodes the tile.
+__device__ __forceinline__ const GemmOp *decode_tile(const GemmOp *ops, int n_ops, int t, int &cursor,
+                                                     Tile &tc) {
+  while (cursor + 1 < n_ops && t >= ops[cursor].tile_base + ops[cursor].n_tiles) ++cursor;
+  const GemmOp *op = ops + cursor;
+  decode_in_op(op, t - op->tile_base, tc);
   return op;
+}
+
+// The op's fields, copied to shared memory by the first threads of the CTA (one 4-byte word each). A barrier of the
+// whole CTA must follow before anyone reads them.
+constexpr int STAGED_OP_BYTES = (int)sizeof(GemmScalars);
+__device__ __forceinline__ void stage_op(GemmScalars *dst, const GemmOp *src, int tid, int threads) {
+  const uint32_t *from = reinterpret_cast<const uint32_t *>(static_cast<const GemmScalars *>(src));
+  uint32_t *to = reinterpret_cast<uint32_t *>(dst);
+  for (int i = tid; i < STAGED_OP_BYTES / 4; i += threads) to[i] = from[i];
 }
 
 static __device__ __noinline__ void raise_timeout(Ctrl *ctrl, const LaunchParams &p, int site, int op, int idx,
@@ -165,7 +177,7 @@ __device__ __forceinline__ bool wait_counter(const unsigned *ctr, unsigned expec
 // is still short is polled (bounded). `rb` is the consumer's 128-row block. `done` remembers, per role and
 // op, which producers have been seen complete as a whole (bit w = dependency w): those are skipped from then
 // on, so the tiles of a long op stop paying for dependencies that were settled during its first wave.
-__device__ __forceinline__ bool wait_deps(const GemmOp *op, int rb, Ctrl *ctrl, const LaunchParams &p, unsigned &done) {
+__device__ __forceinline__ bool wait_deps(const GemmScalars *op, int rb, Ctrl *ctrl, const LaunchParams &p, unsigned &done) {
   bool all = true, looked = false;
   unsigned newly = 0u;
 #pragma unroll

@@ -107,11 +107,10 @@ struct Status {
 // One GEMM as the kernel sees it: C[Mc][Nc] = A . B (+ bias), reduction length Kc.
 // A is "K-major" when its reduction index is contiguous in memory ([Mc][Kc] row-major) and
 // "MN-major" when its Mc index is contiguous ([Kc][Mc] row-major); likewise B with Nc.
-struct alignas(64) GemmOp {
-  CUtensorMap tmA;  // box {32, 128} (K-major) or {32, 32} (MN-major)
-  CUtensorMap tmB;  // box {32, bn}  (K-major) or {32, 32} (MN-major)
-  CUtensorMap tmC;  // output, box {32, 32}: epilogue stores / split-K reduce-adds
-  CUtensorMap tmC2; // second output of the GELU dual store
+// Everything but the tensor maps: a launch of one op copies this part to shared memory when it starts (see
+// stage_op), because a kernel parameter that is read through a pointer costs a round trip of several hundred cycles at
+// every first touch, and the roles of a tile touch dozens of fields one after the other.
+struct alignas(16) GemmScalars {
   int epi_tma;      // 1: the epilogue hands its staged boxes to the copy engine (TMA stores / reduce-adds)
   float *C;
   float *C2;            // gelu(C) when flags & GPT2L_EPI_GELU_DUAL
@@ -180,6 +179,13 @@ struct alignas(64) GemmOp {
   int rb_per_seq;       // DEP_SEQUENCE: 128-row blocks per sequence (T / 128)
   int xform;            // this op needs the operand-transform warps (3xTF32 split or fused column sums)
   RowArgs ra;
+};
+
+struct alignas(64) GemmOp : GemmScalars {
+  CUtensorMap tmA;  // box {32, 128} (K-major) or {32, 32} (MN-major)
+  CUtensorMap tmB;  // box {32, bn}  (K-major) or {32, 32} (MN-major)
+  CUtensorMap tmC;  // output, box {32, 32}: epilogue stores / split-K reduce-adds
+  CUtensorMap tmC2; // second output of the GELU dual store
 };
 
 // tensor maps of one fused-attention pass (attention_flash.cu): K-major views [T rows][64] of one head

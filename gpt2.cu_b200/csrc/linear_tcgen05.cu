@@ -61,7 +61,7 @@ struct RingCfg {
 // Operand transform of one tile: 3xTF32 hi/lo split of every landed stage and / or the bias-gradient
 // column sums of the B blocks. `x` = thread index among the 128 transform threads. Advances `it`.
 template <bool X3>
-__device__ __forceinline__ bool xform_tile(const GemmOp *op, const Tile &tc, uint8_t *ring_ptr, Ctrl *ctrl,
+__device__ __forceinline__ bool xform_tile(const GemmScalars *op, const Tile &tc, uint8_t *ring_ptr, Ctrl *ctrl,
                                            const LaunchParams &p, uint32_t &it, int x, int lane) {
   using R = RingCfg<X3>;
   bool ok = true;
@@ -365,7 +365,7 @@ __device__ __forceinline__ bool attention_tile(const GemmOp *op, const Tile &tc,
   return attention_tile_mode<flash::F_BWD_Q>(op, grb, rb, bh, ring_ptr, ring, ctrl, tmem_base, p, ap, warp, lane);
 }
 
-__device__ __forceinline__ bool is_attention(const GemmOp *op) {
+__device__ __forceinline__ bool is_attention(const GemmScalars *op) {
   return op->op_kind >= OPK_ATTN_FWD && op->op_kind <= OPK_ATTN_BWD_Q;
 }
 
@@ -383,8 +383,8 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
   constexpr int STAGE_STRIDE = R::STAGE_STRIDE;
   constexpr int LO_OFFSET = R::LO_OFFSET;
 
-  const GemmOp *ops = p.ops ? p.ops : &op0;
-  const int n_ops = p.ops ? p.n_ops : 1;
+  const GemmOp *ops = MEGA ? p.ops : &op0;
+  const int n_ops = MEGA ? p.n_ops : 1;
 
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t ring = (raw + 1023u) & ~1023u;
@@ -394,6 +394,26 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
+  // MEGA = false: one op, its fields staged where the step kernel keeps the attention tiles' barriers
+  GemmScalars *staged = reinterpret_cast<GemmScalars *>(reinterpret_cast<uint8_t *>(ctrl) + CTRL_MAIN_BYTES);
+  static_assert(CTRL_MAIN_BYTES + STAGED_OP_BYTES <= SMEM_CTRL_BYTES, "control region too small");
+  if (!MEGA) {
+    stage_op(staged, &op0, tid, NUM_THREADS);
+    if (tid == XFORM_WARP0 * 32) {  // (warps 0 and 1 have the barriers and the tensor memory to set up)
+      prefetch_tensormap(&op0.tmA);
+      prefetch_tensormap(&op0.tmB);
+    }
+  }
+  // decodes tile t: the op's fields (returned) and the place of its tensor maps
+  auto tile_at = [&](int t, int &cursor, Tile &tc, const GemmOp *&maps) -> const GemmScalars * {
+    if (!MEGA) {
+      maps = &op0;
+      decode_in_op(staged, t, tc);
+      return staged;
+    }
+    maps = decode_tile(ops, n_ops, t, cursor, tc);
+    return maps;
+  };
   // MEGA: barrier counts are fixed at their maximum; a party with nothing to do in an op is stood in for
   const bool xf_all = MEGA ? true : (p.xform_active != 0);
 
@@ -438,10 +458,11 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
     unsigned deps_done = 0u;
     for (int t = blockIdx.x; t < p.total_tiles && ok; t += gridDim.x) {
       Tile tc;
-      const GemmOp *op = decode_tile(ops, n_ops, t, cursor, tc);
+      const GemmOp *maps;
+      const GemmScalars *op = tile_at(t, cursor, tc, maps);
       if (MEGA && op->op_kind != OPK_GEMM) {
         // attention tiles take the whole CTA; the row-local ops are the worker warps' alone
-        if (is_attention(op)) ok = attention_tile(op, tc, ring_ptr, ring, ctrl, tmem_base, p, ap, warp, lane);
+        if (is_attention(op)) ok = attention_tile(maps, tc, ring_ptr, ring, ctrl, tmem_base, p, ap, warp, lane);
         continue;
       }
       if (tc.skip) continue;  // every role skips the same tiles, so no barrier phase is consumed
@@ -460,14 +481,18 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
 
       const int m0 = tc.m_tile * BM;
       const int n0 = tc.n_tile * op->bn;
+      // (every field the k-block loop needs, read once: the loop's asm statements would have them reloaded)
       const int a_mn = op->a_mn, b_mn = op->b_mn, bn = op->bn;
+      const bool batched = op->batch > 1, a_3d = op->a_3d != 0, b_3d = op->b_3d != 0;
+      const int op_index = op->op_index;
+      const CUtensorMap *tmA = &maps->tmA, *tmB = &maps->tmB;
       const uint32_t tx_bytes = (uint32_t)(A_TILE_BYTES + bn * BK * 4);
       for (int kb = tc.kb0; kb < tc.kb1; ++kb, ++it) {
         const int s = it % NST;
         const uint32_t ph = (it / NST) & 1u;
         int okl = 1;
         if (lane == 0)
-          okl = wait_bar(smem_u32(&ctrl->empty[s]), ph ^ 1u, ctrl, p, SITE_SMEM_EMPTY, op->op_index, s, 32);
+          okl = wait_bar(smem_u32(&ctrl->empty[s]), ph ^ 1u, ctrl, p, SITE_SMEM_EMPTY, op_index, s, 32);
         ok = __shfl_sync(0xffffffffu, okl, 0) != 0;
         if (!ok) break;
         if (lane == 0) {
@@ -476,27 +501,27 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
           const uint32_t b_dst = a_dst + A_TILE_BYTES;
           mbar_arrive_expect_tx(bar, tx_bytes);
           const int k0 = kb * BK;
-          if (op->batch > 1) {
+          if (batched) {
             // batched operands: two trailing coordinates select the head and the sequence
-            if (!a_mn) tma_load_4d(a_dst, &op->tmA, bar, k0, m0, tc.bh, tc.bb);
-            else tma_load_5d(a_dst, &op->tmA, bar, 0, k0, m0 >> 5, tc.bh, tc.bb);
-            if (!b_mn) tma_load_4d(b_dst, &op->tmB, bar, k0, n0, tc.bh, tc.bb);
-            else tma_load_5d(b_dst, &op->tmB, bar, 0, k0, n0 >> 5, tc.bh, tc.bb);
+            if (!a_mn) tma_load_4d(a_dst, tmA, bar, k0, m0, tc.bh, tc.bb);
+            else tma_load_5d(a_dst, tmA, bar, 0, k0, m0 >> 5, tc.bh, tc.bb);
+            if (!b_mn) tma_load_4d(b_dst, tmB, bar, k0, n0, tc.bh, tc.bb);
+            else tma_load_5d(b_dst, tmB, bar, 0, k0, n0 >> 5, tc.bh, tc.bb);
           } else {
           if (!a_mn) {
-            tma_load_2d(a_dst, &op->tmA, bar, k0, m0);
-          } else if (op->a_3d) {
-            tma_load_3d(a_dst, &op->tmA, bar, 0, k0, m0 >> 5);
+            tma_load_2d(a_dst, tmA, bar, k0, m0);
+          } else if (a_3d) {
+            tma_load_3d(a_dst, tmA, bar, 0, k0, m0 >> 5);
           } else {
 #pragma unroll
-            for (int c = 0; c < BM / 32; ++c) tma_load_2d(a_dst + c * 4096, &op->tmA, bar, m0 + c * 32, k0);
+            for (int c = 0; c < BM / 32; ++c) tma_load_2d(a_dst + c * 4096, tmA, bar, m0 + c * 32, k0);
           }
           if (!b_mn) {
-            tma_load_2d(b_dst, &op->tmB, bar, k0, n0);
-          } else if (op->b_3d) {
-            tma_load_3d(b_dst, &op->tmB, bar, 0, k0, n0 >> 5);
+            tma_load_2d(b_dst, tmB, bar, k0, n0);
+          } else if (b_3d) {
+            tma_load_3d(b_dst, tmB, bar, 0, k0, n0 >> 5);
           } else {
-            for (int c = 0; c < bn / 32; ++c) tma_load_2d(b_dst + c * 4096, &op->tmB, bar, n0 + c * 32, k0);
+            for (int c = 0; c < bn / 32; ++c) tma_load_2d(b_dst + c * 4096, tmB, bar, n0 + c * 32, k0);
           }
           }
         }
@@ -516,18 +541,20 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
     AttnProgress ap;
     int t = blockIdx.x;
     Tile tc;
-    const GemmOp *op = nullptr;
+    const GemmOp *maps = nullptr;
+    const GemmScalars *op = nullptr;
     bool have = t < p.total_tiles;
-    if (have) op = decode_tile(ops, n_ops, t, cursor, tc);
+    if (have) op = tile_at(t, cursor, tc, maps);
     while (have && ok) {
       const int t_next = t + (int)gridDim.x;
       const bool have_next = t_next < p.total_tiles;
       Tile tc_next = tc;
-      const GemmOp *op_next = op;
-      if (have_next) op_next = decode_tile(ops, n_ops, t_next, cursor, tc_next);
+      const GemmOp *maps_next = maps;
+      const GemmScalars *op_next = op;
+      if (have_next) op_next = tile_at(t_next, cursor, tc_next, maps_next);
       if (tc.skip || (MEGA && op->op_kind != OPK_GEMM)) {
-        if (MEGA && is_attention(op)) ok = attention_tile(op, tc, ring_ptr, ring, ctrl, tmem_base, p, ap, warp, lane);
-        t = t_next; tc = tc_next; op = op_next; have = have_next;
+        if (MEGA && is_attention(op)) ok = attention_tile(maps, tc, ring_ptr, ring, ctrl, tmem_base, p, ap, warp, lane);
+        t = t_next; tc = tc_next; op = op_next; maps = maps_next; have = have_next;
         continue;
       }
 
@@ -541,6 +568,7 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
       tc_fence_after();
 
       const uint32_t d_tmem = tmem_base + as * MAX_BN;
+      const int op_index = op->op_index;
       const uint32_t idesc = op->idesc;
       // K-major: 8-row groups 1024 B apart, 128B swizzle; k-step = 32 B inside the row.
       // MN-major: 32-column chunks 4096 B apart (LBO), 4-row k-groups 512 B apart (SBO),
@@ -564,7 +592,7 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
         if (lane == 0) {
           const uint32_t bar = via_ready ? smem_u32(&ctrl->ready[s]) : smem_u32(&ctrl->full[s]);
           okl = wait_bar(bar, via_ready ? ((rdy_par >> s) & 1u) : ph, ctrl, p, via_ready ? SITE_SMEM_READY : SITE_SMEM_FULL,
-                         op->op_index, s);
+                         op_index, s);
         }
         if (via_ready) rdy_par ^= 1u << s;
         ok = __shfl_sync(0xffffffffu, okl, 0) != 0;
@@ -599,6 +627,7 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
       t = t_next;
       tc = tc_next;
       op = op_next;
+      maps = maps_next;
       have = have_next;
       ++tcount;
     }
@@ -611,7 +640,8 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
     bool ok = true;
     for (int t = blockIdx.x; t < p.total_tiles && ok; t += gridDim.x) {
       Tile tc;
-      const GemmOp *op = decode_tile(ops, n_ops, t, cursor, tc);
+      const GemmOp *maps;
+      const GemmScalars *op = tile_at(t, cursor, tc, maps);
       if (tc.skip) continue;
       ok = xform_tile<X3>(op, tc, ring_ptr, ctrl, p, it, x, lane);
     }
@@ -631,12 +661,13 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
     bool ok = true;
     for (int t = blockIdx.x; t < p.total_tiles && ok; t += gridDim.x) {
       Tile tc;
-      const GemmOp *op = decode_tile(ops, n_ops, t, cursor, tc);
+      const GemmOp *maps;
+      const GemmScalars *op = tile_at(t, cursor, tc, maps);
       if (tc.skip) continue;
       // TF32 bias gradient: the helper warps sum their tile's share of g_out while its main loop runs
       if (!X3 && helper && op->colsum != nullptr && op->colsum_spread)
         ok = colsum_global_tile(op, tc, tc.m_tile, tid - XFORM_WARP0 * 32, lane, ctrl, p);
-      if (ok) ok = epilogue_tile<false>(op, tc, tc.m_tile, tcount, helper, n_epi, c_first, 1u, 1u, sbuf,
+      if (ok) ok = epilogue_tile<false>(op, maps, tc, tc.m_tile, tcount, helper, n_epi, c_first, 1u, 1u, sbuf,
                                         n_epi == 1 ? sbuf + EPI_BUF_BYTES : sbuf, tmem_base, ctrl, p, warp, lane);
       ++tcount;
     }
@@ -660,7 +691,8 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
     unsigned deps_done = 0u;
     for (int t = blockIdx.x; t < p.total_tiles && ok; t += gridDim.x) {
       Tile tc;
-      const GemmOp *op = decode_tile(ops, n_ops, t, cursor, tc);
+      const GemmOp *maps;
+      const GemmScalars *op = tile_at(t, cursor, tc, maps);
       if (dep_op != op->op_index) {
         dep_op = op->op_index;
         deps_done = 0u;
@@ -668,18 +700,18 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
       long long t0 = 0;
       if (p.prof && tid == EPI_WARP0 * 32) t0 = globaltimer_ns();
       if (op->op_kind != OPK_GEMM) {
-        if (is_attention(op)) ok = attention_tile(op, tc, ring_ptr, ring, ctrl, tmem_base, p, ap, warp, lane);
-        else ok = row_op_tile(op, tc, w8, lane, scratch, rs, ctrl, p, deps_done);
+        if (is_attention(op)) ok = attention_tile(maps, tc, ring_ptr, ring, ctrl, tmem_base, p, ap, warp, lane);
+        else ok = row_op_tile(maps, tc, w8, lane, scratch, rs, ctrl, p, deps_done);
       } else if (tc.skip) {
         continue;
       } else if (op->xform) {
         if (helper) ok = xform_tile<X3>(op, tc, ring_ptr, ctrl, p, it, x, lane);
-        else ok = epilogue_tile<false>(op, tc, tc.m_tile, tcount, false, 1, 0, 2u, 2u, sbuf, sbuf + EPI_BUF_BYTES, tmem_base, ctrl, p, warp, lane);
+        else ok = epilogue_tile<false>(op, maps, tc, tc.m_tile, tcount, false, 1, 0, 2u, 2u, sbuf, sbuf + EPI_BUF_BYTES, tmem_base, ctrl, p, warp, lane);
         if (!helper) it += (uint32_t)(tc.kb1 - tc.kb0);
         ++tcount;
       } else {
         if (!X3 && helper && op->colsum != nullptr && op->colsum_spread) ok = colsum_global_tile(op, tc, tc.m_tile, x, lane, ctrl, p);
-        if (ok) ok = epilogue_tile<false>(op, tc, tc.m_tile, tcount, helper, 2, helper ? 1 : 0, 1u, 1u, sbuf, sbuf, tmem_base, ctrl, p, warp, lane);
+        if (ok) ok = epilogue_tile<false>(op, maps, tc, tc.m_tile, tcount, helper, 2, helper ? 1 : 0, 1u, 1u, sbuf, sbuf, tmem_base, ctrl, p, warp, lane);
         it += (uint32_t)(tc.kb1 - tc.kb0);
         ++tcount;
       }
@@ -701,8 +733,9 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
     bool ok = true;
     for (int t = blockIdx.x; t < p.total_tiles && ok; t += gridDim.x) {
       Tile tc;
-      const GemmOp *op = decode_tile(ops, n_ops, t, cursor, tc);
-      if (is_attention(op)) ok = attention_tile(op, tc, ring_ptr, ring, ctrl, tmem_base, p, ap, warp, lane);
+      const GemmOp *maps;
+      const GemmScalars *op = tile_at(t, cursor, tc, maps);
+      if (is_attention(op)) ok = attention_tile(maps, tc, ring_ptr, ring, ctrl, tmem_base, p, ap, warp, lane);
     }
   }
 

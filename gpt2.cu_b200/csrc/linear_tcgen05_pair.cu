@@ -65,6 +65,26 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
   const uint32_t rank = cluster_ctarank();       // 0 = leader
   const int pair_id = blockIdx.x >> 1;
   const int n_pairs = gridDim.x >> 1;
+  // a launch of one op keeps the op's fields in shared memory; a list reads them where they are
+  GemmScalars *staged = reinterpret_cast<GemmScalars *>(reinterpret_cast<uint8_t *>(ctrl) + CTRL_MAIN_BYTES);
+  static_assert(CTRL_MAIN_BYTES + STAGED_OP_BYTES <= SMEM_CTRL_BYTES, "control region too small");
+  const bool single = p.ops == nullptr;
+  if (single) {
+    stage_op(staged, &op0, tid, NUM_THREADS);
+    if (tid == XFORM_WARP0 * 32) {
+      prefetch_tensormap(&op0.tmA);
+      prefetch_tensormap(&op0.tmB);
+    }
+  }
+  auto tile_at = [&](int t, int &cursor, Tile &tc, const GemmOp *&maps) -> const GemmScalars * {
+    if (single) {
+      maps = &op0;
+      decode_in_op(staged, t, tc);
+      return staged;
+    }
+    maps = decode_tile(ops, n_ops, t, cursor, tc);
+    return maps;
+  };
   const bool xform = X3 && p.xform_active != 0;  // the transform warps only work in 3xTF32 mode
   // TF32 launches: no warp looks at its own CTA's ring (the transform warps only work in 3xTF32 mode), so the
   // loads of both CTAs complete directly on the leader's full[s]
@@ -102,7 +122,8 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
     bool ok = true;
     for (int t = pair_id; t < p.total_tiles && ok; t += n_pairs) {
       Tile tc;
-      const GemmOp *op = decode_tile(ops, n_ops, t, cursor, tc);
+      const GemmOp *maps;
+      const GemmScalars *op = tile_at(t, cursor, tc, maps);
       const int m_tile = 2 * tc.m_tile + (int)rank;  // this CTA's 128-row block
       bool waited = false;
 #pragma unroll
@@ -128,13 +149,16 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
       const int m0 = m_tile * BM;
       const int n0 = tc.n_tile * op->bn + (int)rank * bh;
       const int a_mn = op->a_mn, b_mn = op->b_mn;
+      const bool a_3d = op->a_3d != 0, b_3d = op->b_3d != 0;
+      const int op_index = op->op_index;
+      const CUtensorMap *tmA = &maps->tmA, *tmB = &maps->tmB;
       const uint32_t tx_bytes = (uint32_t)(A_TILE_BYTES + bh * BK * 4);
       for (int kb = tc.kb0; kb < tc.kb1; ++kb, ++it) {
         const int s = it % NST;
         const uint32_t ph = (it / NST) & 1u;
         int okl = 1;
         if (lane == 0)
-          okl = wait_bar(smem_u32(&ctrl->empty[s]), ph ^ 1u, ctrl, p, SITE_SMEM_EMPTY, op->op_index, s, 32);
+          okl = wait_bar(smem_u32(&ctrl->empty[s]), ph ^ 1u, ctrl, p, SITE_SMEM_EMPTY, op_index, s, 32);
         ok = __shfl_sync(0xffffffffu, okl, 0) != 0;
         if (!ok) break;
         if (lane == 0) {
@@ -148,37 +172,37 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
             const uint32_t bar = mapa_cluster(smem_u32(&ctrl->full[s]), 0);
             if (rank == 0) mbar_arrive_expect_tx(smem_u32(&ctrl->full[s]), 2u * tx_bytes);
             if (!a_mn) {
-              tma_load_2d_pair(a_dst, &op->tmA, bar, k0, m0);
-            } else if (op->a_3d) {
-              tma_load_3d_pair(a_dst, &op->tmA, bar, 0, k0, m0 >> 5);
+              tma_load_2d_pair(a_dst, tmA, bar, k0, m0);
+            } else if (a_3d) {
+              tma_load_3d_pair(a_dst, tmA, bar, 0, k0, m0 >> 5);
             } else {
 #pragma unroll
-              for (int c = 0; c < BM / 32; ++c) tma_load_2d_pair(a_dst + c * 4096, &op->tmA, bar, m0 + c * 32, k0);
+              for (int c = 0; c < BM / 32; ++c) tma_load_2d_pair(a_dst + c * 4096, tmA, bar, m0 + c * 32, k0);
             }
             if (!b_mn) {
-              tma_load_2d_pair(b_dst, &op->tmB, bar, k0, n0);
-            } else if (op->b_3d) {
-              tma_load_3d_pair(b_dst, &op->tmB, bar, 0, k0, n0 >> 5);
+              tma_load_2d_pair(b_dst, tmB, bar, k0, n0);
+            } else if (b_3d) {
+              tma_load_3d_pair(b_dst, tmB, bar, 0, k0, n0 >> 5);
             } else {
-              for (int c = 0; c < bh / 32; ++c) tma_load_2d_pair(b_dst + c * 4096, &op->tmB, bar, n0 + c * 32, k0);
+              for (int c = 0; c < bh / 32; ++c) tma_load_2d_pair(b_dst + c * 4096, tmB, bar, n0 + c * 32, k0);
             }
           } else {
             const uint32_t bar = smem_u32(&ctrl->full[s]);
             mbar_arrive_expect_tx(bar, tx_bytes);
             if (!a_mn) {
-              tma_load_2d(a_dst, &op->tmA, bar, k0, m0);
-            } else if (op->a_3d) {
-              tma_load_3d(a_dst, &op->tmA, bar, 0, k0, m0 >> 5);
+              tma_load_2d(a_dst, tmA, bar, k0, m0);
+            } else if (a_3d) {
+              tma_load_3d(a_dst, tmA, bar, 0, k0, m0 >> 5);
             } else {
 #pragma unroll
-              for (int c = 0; c < BM / 32; ++c) tma_load_2d(a_dst + c * 4096, &op->tmA, bar, m0 + c * 32, k0);
+              for (int c = 0; c < BM / 32; ++c) tma_load_2d(a_dst + c * 4096, tmA, bar, m0 + c * 32, k0);
             }
             if (!b_mn) {
-              tma_load_2d(b_dst, &op->tmB, bar, k0, n0);
-            } else if (op->b_3d) {
-              tma_load_3d(b_dst, &op->tmB, bar, 0, k0, n0 >> 5);
+              tma_load_2d(b_dst, tmB, bar, k0, n0);
+            } else if (b_3d) {
+              tma_load_3d(b_dst, tmB, bar, 0, k0, n0 >> 5);
             } else {
-              for (int c = 0; c < bh / 32; ++c) tma_load_2d(b_dst + c * 4096, &op->tmB, bar, n0 + c * 32, k0);
+              for (int c = 0; c < bh / 32; ++c) tma_load_2d(b_dst + c * 4096, tmB, bar, n0 + c * 32, k0);
             }
           }
         }
@@ -193,7 +217,8 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
     // the same barrier offsets in the peer CTA, as cluster addresses
     for (int t = pair_id; t < p.total_tiles && ok; t += n_pairs, ++tcount) {
       Tile tc;
-      const GemmOp *op = decode_tile(ops, n_ops, t, cursor, tc);
+      const GemmOp *maps;
+      const GemmScalars *op = tile_at(t, cursor, tc, maps);
       const uint32_t as = tcount & 1u;
       const uint32_t aph = (tcount >> 1) & 1u;
       int okl = 1;
@@ -205,6 +230,7 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
       tc_fence_after();
 
       const uint32_t d_tmem = tmem_base + as * MAX_BN;
+      const int op_index = op->op_index;
       const uint32_t idesc = op->idesc;
       const uint64_t hiA = op->a_mn ? smem_desc_hi(4096, 512, 1) : smem_desc_hi(16, 1024, 2);
       const uint64_t hiB = op->b_mn ? smem_desc_hi(4096, 512, 1) : smem_desc_hi(16, 1024, 2);
@@ -218,9 +244,9 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
         if (lane == 0) {
           // TF32: full[s] counts the bytes of both CTAs.
           // 3xTF32: ready counts the transform warps of both CTAs, which implies both rings landed and were split.
-          if (!X3) okl = wait_bar(smem_u32(&ctrl->full[s]), ph, ctrl, p, SITE_SMEM_FULL, op->op_index, s);
+          if (!X3) okl = wait_bar(smem_u32(&ctrl->full[s]), ph, ctrl, p, SITE_SMEM_FULL, op_index, s);
           if (okl && !direct)
-            okl = wait_bar_cluster(smem_u32(&ctrl->ready[s]), ph, ctrl, p, SITE_SMEM_READY, op->op_index, s);
+            okl = wait_bar_cluster(smem_u32(&ctrl->ready[s]), ph, ctrl, p, SITE_SMEM_READY, op_index, s);
         }
         ok = __shfl_sync(0xffffffffu, okl, 0) != 0;
         if (!ok) break;
@@ -269,7 +295,8 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
       bool ok = true;
       for (int t = pair_id; t < p.total_tiles && ok; t += n_pairs) {
         Tile tc;
-        const GemmOp *op = decode_tile(ops, n_ops, t, cursor, tc);
+        const GemmOp *maps;
+        const GemmScalars *op = tile_at(t, cursor, tc, maps);
         const int bh = op->bn >> 1;
         // the bias gradient belongs to tile row 0 (both CTAs of that pair: each sums its half of
         // the columns)
@@ -362,13 +389,14 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
     bool ok = true;
     for (int t = pair_id; t < p.total_tiles && ok; t += n_pairs, ++tcount) {
       Tile tc;
-      const GemmOp *op = decode_tile(ops, n_ops, t, cursor, tc);
+      const GemmOp *maps;
+      const GemmScalars *op = tile_at(t, cursor, tc, maps);
       const int m_tile = 2 * tc.m_tile + (int)rank;
       if (helper) {
         if (!X3 && op->colsum != nullptr && op->colsum_spread && m_tile < op->tiles_m)
           ok = colsum_global_tile(op, tc, m_tile, tid - XFORM_WARP0 * 32, lane, ctrl, p);
       } else {
-        ok = epilogue_tile<true>(op, tc, m_tile, tcount, false, 1, 0, 1u, 1u, sbuf, sbuf + EPI_BUF_BYTES, tmem_base, ctrl,
+        ok = epilogue_tile<true>(op, maps, tc, m_tile, tcount, false, 1, 0, 1u, 1u, sbuf, sbuf + EPI_BUF_BYTES, tmem_base, ctrl,
                                  p, warp, lane);
       }
     }
