@@ -115,16 +115,14 @@ layernorm_forward_vec_kernel(float *out, float *mean, float *rstd, const float *
 
 // g_in[row] += layernorm backward of g_out[row]; g_w / g_b accumulate over rows. A warp owns a row at a
 // time and lane l always owns columns l, l+32, ...: the column sums for g_w / g_b stay in registers
-// across the rows of the block and are combined once (shared memory, then one atomicAdd per column
-// per block).
+// across the rows of the block and are combined once (the warps' sums halve twice through shared memory, then one
+// atomicAdd per column per block). A warp's rows are a chain of dependent reductions, so a short batch gets a
+// row per warp: 256 rows x 768 in blocks of 32 rows took 15.7 us (8 blocks), 5.0 us in blocks of 8.
 template <int K4>  // float4 columns per lane: C <= 128 * K4 (C is a multiple of 4)
 __global__ void __launch_bounds__(256, (K4 <= 6 ? 2 : 1))
 layernorm_backward_kernel(float *g_in, float *g_w, float *g_b, const float *g_out, const float *in, const float *w,
                           const float *mean, const float *rstd, int M, int C, int rows_per_block) {
-  extern __shared__ float sm[];  // [2][C] column sums of this block
-  float *sw = sm, *sb = sm + C;
-  for (int c = threadIdx.x; c < 2 * C; c += blockDim.x) sm[c] = 0.f;
-  __syncthreads();
+  extern __shared__ __align__(16) float sm[];  // [4][C]: column sums of four warps
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   float4 aw[K4], ab[K4];
 #pragma unroll
@@ -138,8 +136,14 @@ layernorm_backward_kernel(float *g_in, float *g_w, float *g_b, const float *g_ou
     const float *x = in + (long long)row * C;
     const float *go = g_out + (long long)row * C;
     const float mu = mean[row], rs = rstd[row];
-    float4 nh[K4], g[K4];
+    float *gi = g_in + (long long)row * C;
+    float4 nh[K4], g[K4], o[K4];
     float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int k = 0; k < K4; ++k) {  // needed last, fetched first: its latency hides behind the two reductions
+      const int c = 4 * (lane + 32 * k);
+      if (c < C) o[k] = *reinterpret_cast<const float4 *>(gi + c);
+    }
 #pragma unroll
     for (int k = 0; k < K4; ++k) {
       const int c = 4 * (lane + 32 * k);
@@ -154,36 +158,44 @@ layernorm_backward_kernel(float *g_in, float *g_w, float *g_b, const float *g_ou
     }
     s1 = warp_sum(s1) / C;
     s2 = warp_sum(s2) / C;
-    float *gi = g_in + (long long)row * C;
 #pragma unroll
     for (int k = 0; k < K4; ++k) {
       const int c = 4 * (lane + 32 * k);
       if (c < C) {
-        float4 o = *reinterpret_cast<float4 *>(gi + c);
         const float4 wv = __ldg(reinterpret_cast<const float4 *>(w + c));
-        o.x += (g[k].x * wv.x - s1 - nh[k].x * s2) * rs;
-        o.y += (g[k].y * wv.y - s1 - nh[k].y * s2) * rs;
-        o.z += (g[k].z * wv.z - s1 - nh[k].z * s2) * rs;
-        o.w += (g[k].w * wv.w - s1 - nh[k].w * s2) * rs;
-        *reinterpret_cast<float4 *>(gi + c) = o;
+        o[k].x += (g[k].x * wv.x - s1 - nh[k].x * s2) * rs;
+        o[k].y += (g[k].y * wv.y - s1 - nh[k].y * s2) * rs;
+        o[k].z += (g[k].z * wv.z - s1 - nh[k].z * s2) * rs;
+        o[k].w += (g[k].w * wv.w - s1 - nh[k].w * s2) * rs;
+        *reinterpret_cast<float4 *>(gi + c) = o[k];
       }
       aw[k].x += g[k].x * nh[k].x; aw[k].y += g[k].y * nh[k].y; aw[k].z += g[k].z * nh[k].z; aw[k].w += g[k].w * nh[k].w;
       ab[k].x += g[k].x; ab[k].y += g[k].y; ab[k].z += g[k].z; ab[k].w += g[k].w;
     }
   }
+  // (eight warps) 4..7 hand their sums to 0..3, then the four are added column by column
+  auto combine = [&](float4 (&v)[K4], float *dst) {
+    float4 *buf = reinterpret_cast<float4 *>(sm + (warp & 3) * C);
+    if (warp >= 4) {
 #pragma unroll
-  for (int k = 0; k < K4; ++k) {
-    const int c = 4 * (lane + 32 * k);
-    if (c < C) {
-      atomicAdd(sw + c, aw[k].x); atomicAdd(sw + c + 1, aw[k].y); atomicAdd(sw + c + 2, aw[k].z); atomicAdd(sw + c + 3, aw[k].w);
-      atomicAdd(sb + c, ab[k].x); atomicAdd(sb + c + 1, ab[k].y); atomicAdd(sb + c + 2, ab[k].z); atomicAdd(sb + c + 3, ab[k].w);
+      for (int k = 0; k < K4; ++k)
+        if (4 * (lane + 32 * k) < C) buf[lane + 32 * k] = v[k];
     }
-  }
-  __syncthreads();
-  for (int c = threadIdx.x; c < C; c += blockDim.x) {
-    atomicAdd(g_w + c, sw[c]);
-    atomicAdd(g_b + c, sb[c]);
-  }
+    __syncthreads();
+    if (warp < 4) {
+#pragma unroll
+      for (int k = 0; k < K4; ++k)
+        if (4 * (lane + 32 * k) < C) {
+          const float4 t = buf[lane + 32 * k];
+          buf[lane + 32 * k] = make_float4(v[k].x + t.x, v[k].y + t.y, v[k].z + t.z, v[k].w + t.w);
+        }
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < C; c += blockDim.x) atomicAdd(dst + c, (sm[c] + sm[C + c]) + (sm[2 * C + c] + sm[3 * C + c]));
+    __syncthreads();
+  };
+  combine(aw, g_w);
+  combine(ab, g_b);
 }
 
 // ------------------------------------------------------------------------------------
@@ -736,7 +748,7 @@ int layernorm_forward(float *out, float *mean, float *rstd, const float *in, con
 int layernorm_backward(float *g_in, float *g_w, float *g_b, const float *g_out, const float *in, const float *w,
                        const float *mean, const float *rstd, int M, int C, cudaStream_t s) {
   // one block per resident slot (two per SM) where there are rows enough: every block then ends at about
-  // the same time, and the column sums meet in global memory only ~300 times instead of M / 32 times
+  // the same time, and the column sums meet in global memory only ~300 times; a row per warp where there are not
   static const int slots = [] {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -744,10 +756,9 @@ int layernorm_backward(float *g_in, float *g_w, float *g_b, const float *g_out, 
       sms = 148;
     return 2 * sms;
   }();
-  int rows_per_block = cdiv(M, slots);
-  if (rows_per_block < 32) rows_per_block = 32;
+  const int rows_per_block = cdiv(cdiv(M, slots), 8) * 8;
   const int blocks = cdiv(M, rows_per_block);
-  const size_t smem = 2 * C * sizeof(float);
+  const size_t smem = 4 * (size_t)C * sizeof(float);
   if (C & 3) return GPT2L_ERR_BAD_ARG;
 #define LN_BWD(K4) layernorm_backward_kernel<K4><<<blocks, 256, smem, s>>>(g_in, g_w, g_b, g_out, in, w, mean, rstd, M, C, rows_per_block)
   if (C <= 128) LN_BWD(1);
