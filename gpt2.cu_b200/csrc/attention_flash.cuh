@@ -75,7 +75,7 @@ struct Cfg {
 
 __device__ __forceinline__ bool f_wait(uint32_t bar, uint32_t parity, FlashCtrl *ctrl, const FlashArgs &a, int site) {
   if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = globaltimer_ns();
+  long long t0 = 0;  // (read only once the wait turns out long, see wait_bar)
   uint32_t spins = 0;
   for (;;) {
     if (mbar_try_wait(bar, parity)) return true;
@@ -85,7 +85,9 @@ __device__ __forceinline__ bool f_wait(uint32_t bar, uint32_t parity, FlashCtrl 
         *reinterpret_cast<volatile int *>(&ctrl->abort) = 1;
         return false;
       }
-      if (globaltimer_ns() - t0 > a.wait_limit_ns) {
+      const long long now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > a.wait_limit_ns) {
         *reinterpret_cast<volatile int *>(&ctrl->abort) = 1;
         if (a.status) atomicCAS(a.status, 0, site);
         if (a.cta_abort) *reinterpret_cast<volatile int *>(a.cta_abort) = 1;
@@ -205,7 +207,7 @@ __device__ __forceinline__ void attn_tile_body(const FlashMaps &maps, const Flas
 
   if (warp == 0) {
     // =============================== TMA producer ===============================
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t bar = smem_u32(&ctrl->fixed_full);
       mbar_arrive_expect_tx(bar, K::NA * TILE_A);  // (waited for with the parity of the tile count)
 #pragma unroll
@@ -258,7 +260,7 @@ __device__ __forceinline__ void attn_tile_body(const FlashMaps &maps, const Flas
     // with %globaltimer) and was what the row work waited for, so the backward modes use two issuing
     // warps: warp 1 the score products, warp 2 the accumulate products. FWD (16 MMAs per step, two CTAs
     // per SM, register-bound) keeps both in warp 1.
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t hiK = smem_desc_hi(16, 1024, 2);     // K-major, 128-byte swizzle
       const uint64_t hiMN = smem_desc_hi(4096, 512, 1);   // MN-major, 32-byte swizzle atoms
       const uint32_t idesc_sc = make_idesc_tf32(FROWS, FC, 0, 0);

@@ -15,7 +15,7 @@ using namespace ptx;
 __device__ __forceinline__ bool wait_bar_cluster(uint32_t bar, uint32_t parity, Ctrl *ctrl, const LaunchParams &p,
                                                  int site, int op, int idx, unsigned backoff_ns = 0) {
   if (mbar_try_wait_cluster(bar, parity)) return true;
-  const long long t0 = globaltimer_ns();
+  long long t0 = 0;
   uint32_t spins = 0;
   for (;;) {
     if (backoff_ns) __nanosleep(backoff_ns);
@@ -26,7 +26,9 @@ __device__ __forceinline__ bool wait_bar_cluster(uint32_t bar, uint32_t parity, 
         *reinterpret_cast<volatile int *>(&ctrl->abort) = 1;
         return false;
       }
-      if (globaltimer_ns() - t0 > p.wait_limit_ns) {
+      const long long now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > p.wait_limit_ns) {
         raise_timeout(ctrl, p, site, op, idx, -1, (int)parity);
         return false;
       }
@@ -175,7 +177,7 @@ __device__ __forceinline__ bool epilogue_tile(const GemmScalars *op, const GemmO
         if (use_tma) {
           // the copy engine takes the box from here: no read-back through the load/store unit and no store
           // instructions, which is what the tensor core's own operand fetches compete with
-          if (lane == 0) {  // the bulk group that read this box last is done reading
+          if (elect_one()) {  // the bulk group that read this box last is done reading
             if (sbuf_alt != sbuf) bulk_wait_read<1>();
             else bulk_wait_read<0>();
           }
@@ -185,7 +187,7 @@ __device__ __forceinline__ bool epilogue_tile(const GemmScalars *op, const GemmO
             st_shared_v4(bx + lane * 128 + ((j ^ (lane & 7)) << 4), v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
           fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0) {
+          if (elect_one()) {
             const CUtensorMap *map = pass == 0 ? &maps->tmC : &maps->tmC2;
             if (op->atomic_out) tma_reduce_add_2d(map, bx, nb, row0);
             else tma_store_2d(map, bx, nb, row0);
@@ -282,7 +284,7 @@ __device__ __forceinline__ bool epilogue_tile(const GemmScalars *op, const GemmO
     }
   }
 
-  if (tma_used && lane == 0) {
+  if (tma_used && elect_one()) {
     // the boxes may be rewritten (or the CTA may exit) only after the copy engine has read them; a published
     // tile must also have landed in global memory
     if (live && pub != 0u && (op->pub_rb_base >= 0 || op->pub_op_ctr >= 0)) {

@@ -9,7 +9,24 @@ namespace g2l {
 
 using namespace ptx;
 
-constexpr int MAX_STAGES = 6;
+constexpr int MAX_STAGES = 8;
+
+// Position in the operand ring: stage and the parity of its current phase.
+struct RingPos {
+  int s = 0;
+  uint32_t ph = 0u;
+  __device__ __forceinline__ void step(int stages) {
+    if (++s == stages) {
+      s = 0;
+      ph ^= 1u;
+    }
+  }
+  __device__ __forceinline__ void skip(int n, int stages) {
+    const int q = s + n;
+    ph ^= (uint32_t)(q / stages) & 1u;
+    s = q % stages;
+  }
+};
 
 // ------------------------------------------------------------------------------------
 // shared-memory control block
@@ -127,7 +144,8 @@ static __device__ __noinline__ void raise_timeout(Ctrl *ctrl, const LaunchParams
 __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, Ctrl *ctrl, const LaunchParams &p,
                                          int site, int op, int idx, unsigned backoff_ns = 0) {
   if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = globaltimer_ns();
+  long long t0 = 0;  // read only once the wait turns out long: a read of %globaltimer takes a good part of a microsecond,
+                     // more than most waits of the ring
   uint32_t spins = 0;
   for (;;) {
     if (backoff_ns) __nanosleep(backoff_ns);
@@ -138,7 +156,9 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, Ctrl *ct
         *reinterpret_cast<volatile int *>(&ctrl->abort) = 1;
         return false;
       }
-      if (globaltimer_ns() - t0 > p.wait_limit_ns) {
+      const long long now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > p.wait_limit_ns) {
         raise_timeout(ctrl, p, site, op, idx, -1, (int)parity);
         return false;
       }
@@ -151,7 +171,7 @@ __device__ __forceinline__ bool wait_counter(const unsigned *ctr, unsigned expec
                                              const LaunchParams &p, int op, int idx) {
   unsigned v = ld_acquire(ctr);
   if (v >= expected) return true;
-  const long long t0 = globaltimer_ns();
+  long long t0 = 0;
   uint32_t spins = 0;
   for (;;) {
     __nanosleep(64);
@@ -163,7 +183,9 @@ __device__ __forceinline__ bool wait_counter(const unsigned *ctr, unsigned expec
         *reinterpret_cast<volatile int *>(&ctrl->abort) = 1;
         return false;
       }
-      if (globaltimer_ns() - t0 > p.wait_limit_ns) {
+      const long long now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > p.wait_limit_ns) {
         raise_timeout(ctrl, p, SITE_DEP_COUNTER, op, idx, (int)v, (int)expected);
         return false;
       }

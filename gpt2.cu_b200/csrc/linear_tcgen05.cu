@@ -51,19 +51,28 @@ using namespace ptx;
 // per-tile bodies of the operand-transform and epilogue roles (shared by the GEMM kernel and the
 // step kernel, which runs them for GEMM tiles between its other ops)
 // ------------------------------------------------------------------------------------
-template <bool X3>
-struct RingCfg {
-  static constexpr int NST = X3 ? STAGES_3X : STAGES_1X;
-  static constexpr int STAGE_STRIDE = X3 ? 2 * STAGE_BYTES : STAGE_BYTES;
-  static constexpr int LO_OFFSET = STAGE_BYTES;  // 3x: lo copies sit behind the hi copies of a stage
+// Shape of the operand ring. The step kernel runs ops of any width through one ring, whose stages are as large as the
+// widest tile's; a launch of one op packs its stages, so that narrow tiles get more of them: 8 for bn = 64, 6 for 128,
+// 4 for 256 (3xTF32, hi and lo copies: 4, 3, 2). A copy takes about a microsecond to land, and with four stages of
+// 24 KiB a k-block of a 128 x 64 tile took 0.44 us, a third more than its MMAs.
+template <bool X3, bool MEGA>
+struct Ring {
+  int stages;
+  uint32_t stride, lo;  // bytes from stage to stage; from a stage's hi copies to its lo copies (3xTF32)
+  __device__ __forceinline__ explicit Ring(int bn) {
+    const uint32_t used = MEGA ? STAGE_BYTES : (uint32_t)(A_TILE_BYTES + bn * BK * 4);
+    lo = used;
+    stride = X3 ? 2u * used : used;
+    const int fit = RING_BYTES / (int)stride;
+    stages = MEGA ? (X3 ? STAGES_3X : STAGES_1X) : (fit < MAX_STAGES ? fit : MAX_STAGES);
+  }
 };
 
 // Operand transform of one tile: 3xTF32 hi/lo split of every landed stage and / or the bias-gradient
-// column sums of the B blocks. `x` = thread index among the 128 transform threads. Advances `it`.
-template <bool X3>
-__device__ __forceinline__ bool xform_tile(const GemmScalars *op, const Tile &tc, uint8_t *ring_ptr, Ctrl *ctrl,
-                                           const LaunchParams &p, uint32_t &it, int x, int lane) {
-  using R = RingCfg<X3>;
+// column sums of the B blocks. `x` = thread index among the 128 transform threads. Advances `pos`.
+template <bool X3, bool MEGA>
+__device__ __forceinline__ bool xform_tile(const GemmScalars *op, const Tile &tc, uint8_t *ring_ptr, const Ring<X3, MEGA> &rg,
+                                           Ctrl *ctrl, const LaunchParams &p, RingPos &pos, int x, int lane) {
   bool ok = true;
   const int bn = op->bn;
   // softmax / cross-entropy backward folded into the operand: the logits become dlogits in shared memory
@@ -91,20 +100,20 @@ __device__ __forceinline__ bool xform_tile(const GemmScalars *op, const Tile &tc
     // TF32 mode: the stages need nothing from these warps (the MMA lane arrives on empty[s] in their place);
     // the column sums, if any, do not go through the ring (colsum_global_tile; every weight gradient is planned
     // with its column sums spread over the tile rows)
-    it += (uint32_t)(tc.kb1 - tc.kb0);
+    pos.skip(tc.kb1 - tc.kb0, rg.stages);
     return has_cs ? colsum_global_tile(op, tc, tc.m_tile, x, lane, ctrl, p) : true;
   }
 
-  for (int kb = tc.kb0; kb < tc.kb1; ++kb, ++it) {
-    const int s = it % R::NST;
-    const uint32_t ph = (it / R::NST) & 1u;
+  for (int kb = tc.kb0; kb < tc.kb1; ++kb, pos.step(rg.stages)) {
+    const int s = pos.s;
+    const uint32_t ph = pos.ph;
     int okl = 1;
     const bool cs_kb = do_colsum && (!spread || (kb % op->tiles_m) == tc.m_tile);
     // (these warps rewrite or sum every stage here, so each is on the ring's critical path: no back-off)
     if (lane == 0) okl = wait_bar(smem_u32(&ctrl->full[s]), ph, ctrl, p, SITE_SMEM_FULL, op->op_index, s);
     ok = __shfl_sync(0xffffffffu, okl, 0) != 0;
     if (!ok) break;
-    uint8_t *stage = ring_ptr + s * R::STAGE_STRIDE;
+    uint8_t *stage = ring_ptr + s * rg.stride;
     if (xmode == 2 && kb == tc.kb0) {
       // only now: the tile's first block has landed, so the producer has seen the tile's dependencies
       // (the row statistics among them) complete
@@ -136,7 +145,7 @@ __device__ __forceinline__ bool xform_tile(const GemmScalars *op, const Tile &tc
           h.x = tf32_round(v.x); h.y = tf32_round(v.y); h.z = tf32_round(v.z); h.w = tf32_round(v.w);
           l.x = v.x - h.x; l.y = v.y - h.y; l.z = v.z - h.z; l.w = v.w - h.w;
           *ptr = h;
-          *reinterpret_cast<float4 *>(reinterpret_cast<uint8_t *>(ptr) + R::LO_OFFSET) = l;
+          *reinterpret_cast<float4 *>(reinterpret_cast<uint8_t *>(ptr) + rg.lo) = l;
         } else {
           *ptr = v;
         }
@@ -169,13 +178,13 @@ __device__ __forceinline__ bool xform_tile(const GemmScalars *op, const Tile &tc
           h.x = tf32_round(v.x); h.y = tf32_round(v.y); h.z = tf32_round(v.z); h.w = tf32_round(v.w);
           l.x = v.x - h.x; l.y = v.y - h.y; l.z = v.z - h.z; l.w = v.w - h.w;
           *ptr = h;
-          *reinterpret_cast<float4 *>(reinterpret_cast<uint8_t *>(ptr) + R::LO_OFFSET) = l;
+          *reinterpret_cast<float4 *>(reinterpret_cast<uint8_t *>(ptr) + rg.lo) = l;
         }
       }
     }
     if (X3) {
       float4 *hi = reinterpret_cast<float4 *>(stage);
-      float4 *lo = reinterpret_cast<float4 *>(stage + R::LO_OFFSET);
+      float4 *lo = reinterpret_cast<float4 *>(stage + rg.lo);
       // what is left to split linearly: A (unless its rows were rewritten above) and a K-major B
       const int lin_lo = xmode == 2 ? (A_TILE_BYTES >> 4) : 0;
       const int lin_f4 = walk_b ? (A_TILE_BYTES >> 4) : stage_f4;
@@ -214,6 +223,114 @@ __device__ __forceinline__ bool xform_tile(const GemmScalars *op, const Tile &tc
       }
     }
   }
+  return true;
+}
+
+// The loads of one tile's k-blocks and its MMAs. Each runs in ONE thread of its warp from the first k-block to the last:
+// with the warp in step around every k-block (poll in lane 0, a shuffle of the verdict, a branch to one lane) the issuer
+// took 650 cycles a k-block whatever the tile's width, where the four MMAs of a 128 x 256 tile need 500 and those of a
+// 128 x 64 tile 200.
+template <bool X3, bool MEGA>
+__device__ __forceinline__ bool load_tile(const GemmScalars *op, const GemmOp *maps, const Tile &tc, const Ring<X3, MEGA> &rg,
+                                          uint32_t ring, Ctrl *ctrl, const LaunchParams &p, RingPos pos) {
+  const int m0 = tc.m_tile * BM;
+  const int n0 = tc.n_tile * op->bn;
+  // (every field the k-block loop needs, read once: the loop's asm statements would have them reloaded)
+  const int a_mn = op->a_mn, b_mn = op->b_mn, bn = op->bn;
+  const bool batched = op->batch > 1, a_3d = op->a_3d != 0, b_3d = op->b_3d != 0;
+  const int op_index = op->op_index;
+  const CUtensorMap *tmA = &maps->tmA, *tmB = &maps->tmB;
+  const uint32_t tx_bytes = (uint32_t)(A_TILE_BYTES + bn * BK * 4);
+  for (int kb = tc.kb0; kb < tc.kb1; ++kb, pos.step(rg.stages)) {
+    const int s = pos.s;
+    if (!wait_bar(smem_u32(&ctrl->empty[s]), pos.ph ^ 1u, ctrl, p, SITE_SMEM_EMPTY, op_index, s, 32)) return false;
+    const uint32_t bar = smem_u32(&ctrl->full[s]);
+    const uint32_t a_dst = ring + s * rg.stride;
+    const uint32_t b_dst = a_dst + A_TILE_BYTES;
+    mbar_arrive_expect_tx(bar, tx_bytes);
+    const int k0 = kb * BK;
+    if (batched) {
+      // batched operands: two trailing coordinates select the head and the sequence
+      if (!a_mn) tma_load_4d(a_dst, tmA, bar, k0, m0, tc.bh, tc.bb);
+      else tma_load_5d(a_dst, tmA, bar, 0, k0, m0 >> 5, tc.bh, tc.bb);
+      if (!b_mn) tma_load_4d(b_dst, tmB, bar, k0, n0, tc.bh, tc.bb);
+      else tma_load_5d(b_dst, tmB, bar, 0, k0, n0 >> 5, tc.bh, tc.bb);
+      continue;
+    }
+    if (!a_mn) {
+      tma_load_2d(a_dst, tmA, bar, k0, m0);
+    } else if (a_3d) {
+      tma_load_3d(a_dst, tmA, bar, 0, k0, m0 >> 5);
+    } else {
+#pragma unroll
+      for (int c = 0; c < BM / 32; ++c) tma_load_2d(a_dst + c * 4096, tmA, bar, m0 + c * 32, k0);
+    }
+    if (!b_mn) {
+      tma_load_2d(b_dst, tmB, bar, k0, n0);
+    } else if (b_3d) {
+      tma_load_3d(b_dst, tmB, bar, 0, k0, n0 >> 5);
+    } else {
+      for (int c = 0; c < bn / 32; ++c) tma_load_2d(b_dst + c * 4096, tmB, bar, n0 + c * 32, k0);
+    }
+  }
+  return true;
+}
+
+template <bool X3, bool MEGA>
+__device__ __forceinline__ bool mma_tile(const GemmScalars *op, const Tile &tc, const Ring<X3, MEGA> &rg, uint32_t ring, Ctrl *ctrl,
+                                         const LaunchParams &p, RingPos pos, uint32_t rdy_par, uint32_t tmem_base,
+                                         uint32_t tcount) {
+  const uint32_t as = tcount & 1u;
+  const uint32_t aph = (tcount >> 1) & 1u;
+  const int op_index = op->op_index;
+  if (!wait_bar(smem_u32(&ctrl->tmem_empty[as]), aph ^ 1u, ctrl, p, SITE_TMEM_EMPTY, op_index, as, 32)) return false;
+  tc_fence_after();  // the epilogue's reads of this accumulator are done
+
+  const uint32_t d_tmem = tmem_base + as * MAX_BN;
+  const uint32_t idesc = op->idesc;
+  // K-major: 8-row groups 1024 B apart, 128B swizzle; k-step = 32 B inside the row.
+  // MN-major: 32-column chunks 4096 B apart (LBO), 4-row k-groups 512 B apart (SBO),
+  //           128B swizzle on 32-byte atoms; k-step = 8 rows = 1024 B.
+  const uint64_t hiA = op->a_mn ? smem_desc_hi(4096, 512, 1) : smem_desc_hi(16, 1024, 2);
+  const uint64_t hiB = op->b_mn ? smem_desc_hi(4096, 512, 1) : smem_desc_hi(16, 1024, 2);
+  const uint32_t stepA = op->a_mn ? 1024u : 32u;
+  const uint32_t stepB = op->b_mn ? 1024u : 32u;
+  // The transform warps' share of empty[s] is left to us wherever they do not touch the stages: in the step
+  // kernel for every op that needs no operand transform, and in any TF32 launch whose barriers count them
+  // (they rewrite stages only in 3xTF32 mode and for the fused cross-entropy; the bias gradient is read
+  // beside the ring).
+  const bool via_ready = X3 || op->xent_mode >= 2;  // the transform warps hand the stage over
+  const bool xf_counted = MEGA || p.xform_active != 0;
+  const bool stand_in = xf_counted && !((MEGA ? (op->xform != 0) : (p.xform_active != 0)) && via_ready);
+
+  for (int kb = tc.kb0; kb < tc.kb1; ++kb, pos.step(rg.stages)) {
+    const int s = pos.s;
+    // (in the step kernel only some ops' k-blocks go through `ready`, so its phases do not follow the ring position)
+    const uint32_t bar = via_ready ? smem_u32(&ctrl->ready[s]) : smem_u32(&ctrl->full[s]);
+    const uint32_t par = MEGA && via_ready ? (rdy_par >> s) & 1u : pos.ph;
+    if (!wait_bar(bar, par, ctrl, p, via_ready ? SITE_SMEM_READY : SITE_SMEM_FULL, op_index, s)) return false;
+    if (MEGA && via_ready) rdy_par ^= 1u << s;
+    const uint32_t a_addr = ring + s * rg.stride;
+    const uint32_t b_addr = a_addr + A_TILE_BYTES;
+#pragma unroll
+    for (int ks = 0; ks < BK / UMMA_K; ++ks) {
+      const uint32_t acc = (kb > tc.kb0 || ks > 0) ? 1u : 0u;
+      const uint64_t da = smem_desc(hiA, a_addr + ks * stepA);
+      const uint64_t db = smem_desc(hiB, b_addr + ks * stepB);
+      if (X3) {
+        const uint64_t da_lo = smem_desc(hiA, a_addr + rg.lo + ks * stepA);
+        const uint64_t db_lo = smem_desc(hiB, b_addr + rg.lo + ks * stepB);
+        mma_tf32(d_tmem, da_lo, db, idesc, acc);  // small terms first
+        mma_tf32(d_tmem, da, db_lo, idesc, 1u);
+        mma_tf32(d_tmem, da, db, idesc, 1u);
+      } else {
+        mma_tf32(d_tmem, da, db, idesc, acc);
+      }
+    }
+    mma_commit(smem_u32(&ctrl->empty[s]));  // frees the stage once these MMAs have read it
+    if (stand_in) mbar_arrive_cnt(smem_u32(&ctrl->empty[s]), NUM_XFORM_WARPS);
+  }
+  mma_commit(smem_u32(&ctrl->tmem_full[as]));
   return true;
 }
 
@@ -378,10 +495,6 @@ template <bool X3, bool MEGA>
 __global__ void __launch_bounds__(MEGA ? STEP_THREADS : NUM_THREADS, 1)
 gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParams p) {
   extern __shared__ uint8_t smem_raw[];
-  using R = RingCfg<X3>;
-  constexpr int NST = R::NST;
-  constexpr int STAGE_STRIDE = R::STAGE_STRIDE;
-  constexpr int LO_OFFSET = R::LO_OFFSET;
 
   const GemmOp *ops = MEGA ? p.ops : &op0;
   const int n_ops = MEGA ? p.n_ops : 1;
@@ -402,6 +515,7 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
     if (tid == XFORM_WARP0 * 32) {  // (warps 0 and 1 have the barriers and the tensor memory to set up)
       prefetch_tensormap(&op0.tmA);
       prefetch_tensormap(&op0.tmB);
+      if (op0.epi_tma) prefetch_tensormap(&op0.tmC);
     }
   }
   // decodes tile t: the op's fields (returned) and the place of its tensor maps
@@ -418,7 +532,7 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
   const bool xf_all = MEGA ? true : (p.xform_active != 0);
 
   if (tid == 0) {
-    for (int s = 0; s < STAGES_1X; ++s) {
+    for (int s = 0; s < MAX_STAGES; ++s) {
       mbar_init(smem_u32(&ctrl->full[s]), 1);
       mbar_init(smem_u32(&ctrl->empty[s]), 1 + (xf_all ? NUM_XFORM_WARPS : 0));
       mbar_init(smem_u32(&ctrl->ready[s]), NUM_XFORM_WARPS);
@@ -447,11 +561,12 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(&ctrl->tmem_base);
+  const Ring<X3, MEGA> rg(MEGA ? 0 : staged->bn);
 
   if (warp == 0) {
     // =============================== TMA producer ===============================
     int cursor = 0;
-    uint32_t it = 0;
+    RingPos pos;
     bool ok = true;
     AttnProgress ap;
     int dep_op = -1;
@@ -479,61 +594,18 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
         fence_proxy_async_all();  // producers wrote with plain stores; TMA reads next
       }
 
-      const int m0 = tc.m_tile * BM;
-      const int n0 = tc.n_tile * op->bn;
-      // (every field the k-block loop needs, read once: the loop's asm statements would have them reloaded)
-      const int a_mn = op->a_mn, b_mn = op->b_mn, bn = op->bn;
-      const bool batched = op->batch > 1, a_3d = op->a_3d != 0, b_3d = op->b_3d != 0;
-      const int op_index = op->op_index;
-      const CUtensorMap *tmA = &maps->tmA, *tmB = &maps->tmB;
-      const uint32_t tx_bytes = (uint32_t)(A_TILE_BYTES + bn * BK * 4);
-      for (int kb = tc.kb0; kb < tc.kb1; ++kb, ++it) {
-        const int s = it % NST;
-        const uint32_t ph = (it / NST) & 1u;
-        int okl = 1;
-        if (lane == 0)
-          okl = wait_bar(smem_u32(&ctrl->empty[s]), ph ^ 1u, ctrl, p, SITE_SMEM_EMPTY, op_index, s, 32);
-        ok = __shfl_sync(0xffffffffu, okl, 0) != 0;
-        if (!ok) break;
-        if (lane == 0) {
-          const uint32_t bar = smem_u32(&ctrl->full[s]);
-          const uint32_t a_dst = ring + s * STAGE_STRIDE;
-          const uint32_t b_dst = a_dst + A_TILE_BYTES;
-          mbar_arrive_expect_tx(bar, tx_bytes);
-          const int k0 = kb * BK;
-          if (batched) {
-            // batched operands: two trailing coordinates select the head and the sequence
-            if (!a_mn) tma_load_4d(a_dst, tmA, bar, k0, m0, tc.bh, tc.bb);
-            else tma_load_5d(a_dst, tmA, bar, 0, k0, m0 >> 5, tc.bh, tc.bb);
-            if (!b_mn) tma_load_4d(b_dst, tmB, bar, k0, n0, tc.bh, tc.bb);
-            else tma_load_5d(b_dst, tmB, bar, 0, k0, n0 >> 5, tc.bh, tc.bb);
-          } else {
-          if (!a_mn) {
-            tma_load_2d(a_dst, tmA, bar, k0, m0);
-          } else if (a_3d) {
-            tma_load_3d(a_dst, tmA, bar, 0, k0, m0 >> 5);
-          } else {
-#pragma unroll
-            for (int c = 0; c < BM / 32; ++c) tma_load_2d(a_dst + c * 4096, tmA, bar, m0 + c * 32, k0);
-          }
-          if (!b_mn) {
-            tma_load_2d(b_dst, tmB, bar, k0, n0);
-          } else if (b_3d) {
-            tma_load_3d(b_dst, tmB, bar, 0, k0, n0 >> 5);
-          } else {
-            for (int c = 0; c < bn / 32; ++c) tma_load_2d(b_dst + c * 4096, tmB, bar, n0 + c * 32, k0);
-          }
-          }
-        }
-        __syncwarp();
-      }
+      int okl = 1;
+      if (elect_one()) okl = load_tile<X3, MEGA>(op, maps, tc, rg, ring, ctrl, p, pos) ? 1 : 0;
+      ok = __all_sync(0xffffffffu, okl) != 0;
+      pos.skip(tc.kb1 - tc.kb0, rg.stages);
     }
   } else if (warp == 1) {
     // =============================== MMA issuer ===============================
     // The next tile is decoded while the current one is being issued: at a tile boundary the
     // tensor pipe holds less than a k-block of queued work, so nothing slow may sit there.
     int cursor = 0;
-    uint32_t it = 0, tcount = 0;
+    RingPos pos;
+    uint32_t tcount = 0;
     // one parity bit per stage for the `ready` barriers: only k-blocks whose stage is rewritten (3xTF32
     // split, logits -> dlogits) go through them, so their phases do not follow the ring position
     uint32_t rdy_par = 0u;
@@ -558,72 +630,15 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
         continue;
       }
 
-      const uint32_t as = tcount & 1u;
-      const uint32_t aph = (tcount >> 1) & 1u;
       int okl = 1;
-      if (lane == 0)
-        okl = wait_bar(smem_u32(&ctrl->tmem_empty[as]), aph ^ 1u, ctrl, p, SITE_TMEM_EMPTY, op->op_index, as, 32);
-      ok = __shfl_sync(0xffffffffu, okl, 0) != 0;
+      if (elect_one()) okl = mma_tile<X3, MEGA>(op, tc, rg, ring, ctrl, p, pos, rdy_par, tmem_base, tcount) ? 1 : 0;
+      ok = __all_sync(0xffffffffu, okl) != 0;
       if (!ok) break;
-      tc_fence_after();
-
-      const uint32_t d_tmem = tmem_base + as * MAX_BN;
-      const int op_index = op->op_index;
-      const uint32_t idesc = op->idesc;
-      // K-major: 8-row groups 1024 B apart, 128B swizzle; k-step = 32 B inside the row.
-      // MN-major: 32-column chunks 4096 B apart (LBO), 4-row k-groups 512 B apart (SBO),
-      //           128B swizzle on 32-byte atoms; k-step = 8 rows = 1024 B.
-      const uint64_t hiA = op->a_mn ? smem_desc_hi(4096, 512, 1) : smem_desc_hi(16, 1024, 2);
-      const uint64_t hiB = op->b_mn ? smem_desc_hi(4096, 512, 1) : smem_desc_hi(16, 1024, 2);
-      const uint32_t stepA = op->a_mn ? 1024u : 32u;
-      const uint32_t stepB = op->b_mn ? 1024u : 32u;
-      // The transform warps' share of empty[s] is left to us wherever they do not touch the stages: in the step
-      // kernel for every op that needs no operand transform, and in any TF32 launch whose barriers count them
-      // (they rewrite stages only in 3xTF32 mode and for the fused cross-entropy; the bias gradient is read
-      // beside the ring).
-      const bool via_ready = X3 || op->xent_mode >= 2;  // the transform warps hand the stage over
-      const bool xf_counted = MEGA || p.xform_active != 0;
-      const bool stand_in = xf_counted && !((MEGA ? (op->xform != 0) : (p.xform_active != 0)) && via_ready);
-
-      for (int kb = tc.kb0; kb < tc.kb1; ++kb, ++it) {
-        const int s = it % NST;
-        const uint32_t ph = (it / NST) & 1u;
-        okl = 1;
-        if (lane == 0) {
-          const uint32_t bar = via_ready ? smem_u32(&ctrl->ready[s]) : smem_u32(&ctrl->full[s]);
-          okl = wait_bar(bar, via_ready ? ((rdy_par >> s) & 1u) : ph, ctrl, p, via_ready ? SITE_SMEM_READY : SITE_SMEM_FULL,
-                         op_index, s);
-        }
-        if (via_ready) rdy_par ^= 1u << s;
-        ok = __shfl_sync(0xffffffffu, okl, 0) != 0;
-        if (!ok) break;
-        tc_fence_after();
-        if (lane == 0) {
-          const uint32_t a_addr = ring + s * STAGE_STRIDE;
-          const uint32_t b_addr = a_addr + A_TILE_BYTES;
-#pragma unroll
-          for (int ks = 0; ks < BK / UMMA_K; ++ks) {
-            const uint32_t acc = (kb > tc.kb0 || ks > 0) ? 1u : 0u;
-            const uint64_t da = smem_desc(hiA, a_addr + ks * stepA);
-            const uint64_t db = smem_desc(hiB, b_addr + ks * stepB);
-            if (X3) {
-              const uint64_t da_lo = smem_desc(hiA, a_addr + LO_OFFSET + ks * stepA);
-              const uint64_t db_lo = smem_desc(hiB, b_addr + LO_OFFSET + ks * stepB);
-              mma_tf32(d_tmem, da_lo, db, idesc, acc);  // small terms first
-              mma_tf32(d_tmem, da, db_lo, idesc, 1u);
-              mma_tf32(d_tmem, da, db, idesc, 1u);
-            } else {
-              mma_tf32(d_tmem, da, db, idesc, acc);
-            }
-          }
-          mma_commit(smem_u32(&ctrl->empty[s]));  // frees the stage once these MMAs have read it
-          if (stand_in) mbar_arrive_cnt(smem_u32(&ctrl->empty[s]), NUM_XFORM_WARPS);
-        }
-        __syncwarp();
+      if (MEGA && (X3 || op->xent_mode >= 2)) {
+        for (int kb = tc.kb0; kb < tc.kb1; ++kb, pos.step(rg.stages)) rdy_par ^= 1u << pos.s;
+      } else {
+        pos.skip(tc.kb1 - tc.kb0, rg.stages);
       }
-      if (!ok) break;
-      if (lane == 0) mma_commit(smem_u32(&ctrl->tmem_full[as]));
-      __syncwarp();
       t = t_next;
       tc = tc_next;
       op = op_next;
@@ -636,14 +651,14 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
     // (in launches where no op needs a split or a column sum these warps join the epilogue instead)
     const int x = tid - XFORM_WARP0 * 32;  // 0..127
     int cursor = 0;
-    uint32_t it = 0;
+    RingPos pos;
     bool ok = true;
     for (int t = blockIdx.x; t < p.total_tiles && ok; t += gridDim.x) {
       Tile tc;
       const GemmOp *maps;
       const GemmScalars *op = tile_at(t, cursor, tc, maps);
       if (tc.skip) continue;
-      ok = xform_tile<X3>(op, tc, ring_ptr, ctrl, p, it, x, lane);
+      ok = xform_tile<X3, MEGA>(op, tc, ring_ptr, rg, ctrl, p, pos, x, lane);
     }
   } else if (!MEGA) {
     // =============================== epilogue ===============================
@@ -685,7 +700,8 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
     RowSync rs = {smem_u32(&ctrl->row_bar), 0u, ctrl};
     AttnProgress ap;
     int cursor = 0;
-    uint32_t it = 0, tcount = 0;
+    RingPos pos;
+    uint32_t tcount = 0;
     bool ok = true;
     int dep_op = -1;
     unsigned deps_done = 0u;
@@ -705,14 +721,14 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
       } else if (tc.skip) {
         continue;
       } else if (op->xform) {
-        if (helper) ok = xform_tile<X3>(op, tc, ring_ptr, ctrl, p, it, x, lane);
+        if (helper) ok = xform_tile<X3, MEGA>(op, tc, ring_ptr, rg, ctrl, p, pos, x, lane);
         else ok = epilogue_tile<false>(op, maps, tc, tc.m_tile, tcount, false, 1, 0, 2u, 2u, sbuf, sbuf + EPI_BUF_BYTES, tmem_base, ctrl, p, warp, lane);
-        if (!helper) it += (uint32_t)(tc.kb1 - tc.kb0);
+        if (!helper) pos.skip(tc.kb1 - tc.kb0, rg.stages);
         ++tcount;
       } else {
         if (!X3 && helper && op->colsum != nullptr && op->colsum_spread) ok = colsum_global_tile(op, tc, tc.m_tile, x, lane, ctrl, p);
         if (ok) ok = epilogue_tile<false>(op, maps, tc, tc.m_tile, tcount, helper, 2, helper ? 1 : 0, 1u, 1u, sbuf, sbuf, tmem_base, ctrl, p, warp, lane);
-        it += (uint32_t)(tc.kb1 - tc.kb0);
+        pos.skip(tc.kb1 - tc.kb0, rg.stages);
         ++tcount;
       }
       if (p.prof && tid == EPI_WARP0 * 32) {

@@ -74,6 +74,7 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
     if (tid == XFORM_WARP0 * 32) {
       prefetch_tensormap(&op0.tmA);
       prefetch_tensormap(&op0.tmB);
+      if (op0.epi_tma) prefetch_tensormap(&op0.tmC);
     }
   }
   auto tile_at = [&](int t, int &cursor, Tile &tc, const GemmOp *&maps) -> const GemmScalars * {
@@ -118,7 +119,7 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
   if (warp == 0) {
     // =============================== TMA producer (both CTAs) ===============================
     int cursor = 0;
-    uint32_t it = 0;
+    RingPos pos;
     bool ok = true;
     for (int t = pair_id; t < p.total_tiles && ok; t += n_pairs) {
       Tile tc;
@@ -153,15 +154,16 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
       const int op_index = op->op_index;
       const CUtensorMap *tmA = &maps->tmA, *tmB = &maps->tmB;
       const uint32_t tx_bytes = (uint32_t)(A_TILE_BYTES + bh * BK * 4);
-      for (int kb = tc.kb0; kb < tc.kb1; ++kb, ++it) {
-        const int s = it % NST;
-        const uint32_t ph = (it / NST) & 1u;
-        int okl = 1;
-        if (lane == 0)
-          okl = wait_bar(smem_u32(&ctrl->empty[s]), ph ^ 1u, ctrl, p, SITE_SMEM_EMPTY, op_index, s, 32);
-        ok = __shfl_sync(0xffffffffu, okl, 0) != 0;
-        if (!ok) break;
-        if (lane == 0) {
+      // (one thread for all k-blocks of the tile, here and in the issuer: see load_tile in linear_tcgen05.cu)
+      int okl = 1;
+      if (elect_one()) {
+        RingPos at = pos;
+        for (int kb = tc.kb0; kb < tc.kb1; ++kb, at.step(NST)) {
+          const int s = at.s;
+          if (!wait_bar(smem_u32(&ctrl->empty[s]), at.ph ^ 1u, ctrl, p, SITE_SMEM_EMPTY, op_index, s, 32)) {
+            okl = 0;
+            break;
+          }
           const uint32_t a_dst = ring + s * STAGE_STRIDE;
           const uint32_t b_dst = a_dst + A_TILE_BYTES;
           const int k0 = kb * BK;
@@ -206,52 +208,41 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
             }
           }
         }
-        __syncwarp();
       }
+      ok = __all_sync(0xffffffffu, okl) != 0;
+      pos.skip(tc.kb1 - tc.kb0, NST);
     }
   } else if (warp == 1 && rank == 0) {
     // =============================== MMA issuer (leader) ===============================
     int cursor = 0;
-    uint32_t it = 0, tcount = 0;
+    RingPos pos;
+    uint32_t tcount = 0;
     bool ok = true;
-    // the same barrier offsets in the peer CTA, as cluster addresses
     for (int t = pair_id; t < p.total_tiles && ok; t += n_pairs, ++tcount) {
       Tile tc;
       const GemmOp *maps;
       const GemmScalars *op = tile_at(t, cursor, tc, maps);
-      const uint32_t as = tcount & 1u;
-      const uint32_t aph = (tcount >> 1) & 1u;
       int okl = 1;
-      if (lane == 0)
-        okl = wait_bar_cluster(smem_u32(&ctrl->tmem_empty[as]), aph ^ 1u, ctrl, p, SITE_TMEM_EMPTY, op->op_index,
-                               as, 32);
-      ok = __shfl_sync(0xffffffffu, okl, 0) != 0;
-      if (!ok) break;
-      tc_fence_after();
-
-      const uint32_t d_tmem = tmem_base + as * MAX_BN;
-      const int op_index = op->op_index;
-      const uint32_t idesc = op->idesc;
-      const uint64_t hiA = op->a_mn ? smem_desc_hi(4096, 512, 1) : smem_desc_hi(16, 1024, 2);
-      const uint64_t hiB = op->b_mn ? smem_desc_hi(4096, 512, 1) : smem_desc_hi(16, 1024, 2);
-      const uint32_t stepA = op->a_mn ? 1024u : 32u;
-      const uint32_t stepB = op->b_mn ? 1024u : 32u;
-
-      for (int kb = tc.kb0; kb < tc.kb1; ++kb, ++it) {
-        const int s = it % NST;
-        const uint32_t ph = (it / NST) & 1u;
-        okl = 1;
-        if (lane == 0) {
+      if (elect_one()) {
+        const uint32_t as = tcount & 1u;
+        const uint32_t aph = (tcount >> 1) & 1u;
+        const int op_index = op->op_index;
+        const uint32_t d_tmem = tmem_base + as * MAX_BN;
+        const uint32_t idesc = op->idesc;
+        const uint64_t hiA = op->a_mn ? smem_desc_hi(4096, 512, 1) : smem_desc_hi(16, 1024, 2);
+        const uint64_t hiB = op->b_mn ? smem_desc_hi(4096, 512, 1) : smem_desc_hi(16, 1024, 2);
+        const uint32_t stepA = op->a_mn ? 1024u : 32u;
+        const uint32_t stepB = op->b_mn ? 1024u : 32u;
+        RingPos at = pos;
+        okl = wait_bar_cluster(smem_u32(&ctrl->tmem_empty[as]), aph ^ 1u, ctrl, p, SITE_TMEM_EMPTY, op_index, as, 32) ? 1 : 0;
+        tc_fence_after();  // the epilogues' reads of this accumulator are done
+        for (int kb = tc.kb0; kb < tc.kb1 && okl; ++kb, at.step(NST)) {
+          const int s = at.s;
           // TF32: full[s] counts the bytes of both CTAs.
           // 3xTF32: ready counts the transform warps of both CTAs, which implies both rings landed and were split.
-          if (!X3) okl = wait_bar(smem_u32(&ctrl->full[s]), ph, ctrl, p, SITE_SMEM_FULL, op_index, s);
-          if (okl && !direct)
-            okl = wait_bar_cluster(smem_u32(&ctrl->ready[s]), ph, ctrl, p, SITE_SMEM_READY, op_index, s);
-        }
-        ok = __shfl_sync(0xffffffffu, okl, 0) != 0;
-        if (!ok) break;
-        tc_fence_after();
-        if (lane == 0) {
+          okl = (X3 ? wait_bar_cluster(smem_u32(&ctrl->ready[s]), at.ph, ctrl, p, SITE_SMEM_READY, op_index, s)
+                    : wait_bar(smem_u32(&ctrl->full[s]), at.ph, ctrl, p, SITE_SMEM_FULL, op_index, s)) ? 1 : 0;
+          if (!okl) break;
           const uint32_t a_addr = ring + s * STAGE_STRIDE;
           const uint32_t b_addr = a_addr + A_TILE_BYTES;
 #pragma unroll
@@ -274,15 +265,14 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
           mma_commit_pair(mapa_cluster(e, 0));
           mma_commit_pair(mapa_cluster(e, 1));
         }
-        __syncwarp();
+        if (okl) {
+          const uint32_t f = smem_u32(&ctrl->tmem_full[as]);
+          mma_commit_pair(mapa_cluster(f, 0));
+          mma_commit_pair(mapa_cluster(f, 1));
+        }
       }
-      if (!ok) break;
-      if (lane == 0) {
-        const uint32_t f = smem_u32(&ctrl->tmem_full[as]);
-        mma_commit_pair(mapa_cluster(f, 0));
-        mma_commit_pair(mapa_cluster(f, 1));
-      }
-      __syncwarp();
+      ok = __all_sync(0xffffffffu, okl) != 0;
+      pos.skip(tc.kb1 - tc.kb0, NST);
     }
   } else if (warp == 1) {
     // (the peer CTA issues no MMAs: its warp 1 only allocates and frees tensor memory)
