@@ -46,18 +46,6 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const float *src, bool l
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(live ? 4 : 0) : "memory");
 }
 
-// two fp32 values in a register pair: {x, x}, and d = a * b + c per half (each half rounded as fmaf rounds it)
-__device__ __forceinline__ unsigned long long both(float x) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-
 // One operand's slab: EXT rows (i or j) by SK k. KC: contiguous in k (a warp copies 8 k of 4 rows, which the row
 // pitch of 4 mod 32 banks stores without conflict); else contiguous in the row index.
 template <int EXT, bool KC>
@@ -159,7 +147,7 @@ gpt2_linear_simt_kernel(float *__restrict__ c, const float *__restrict__ a, cons
 #pragma unroll
       for (int h = 0; h < TM / 4; ++h) {
         const float4 v = *reinterpret_cast<const float4 *>(sa + k * G::LDA + 16 * h);
-        av[4 * h] = both(v.x); av[4 * h + 1] = both(v.y); av[4 * h + 2] = both(v.z); av[4 * h + 3] = both(v.w);
+        av[4 * h] = ptx::both(v.x); av[4 * h + 1] = ptx::both(v.y); av[4 * h + 2] = ptx::both(v.z); av[4 * h + 3] = ptx::both(v.w);
       }
 #pragma unroll
       for (int h = 0; h < TN / 4; ++h) {
@@ -169,7 +157,7 @@ gpt2_linear_simt_kernel(float *__restrict__ c, const float *__restrict__ a, cons
 #pragma unroll
       for (int u = 0; u < TM; ++u)
 #pragma unroll
-        for (int v = 0; v < TN / 2; ++v) acc[u][v] = fma2(av[u], bv[v], acc[u][v]);
+        for (int v = 0; v < TN / 2; ++v) acc[u][v] = ptx::fma2(av[u], bv[v], acc[u][v]);
     }
     stage = stage + 1 == SIMT_STAGES ? 0 : stage + 1;
   }

@@ -304,6 +304,19 @@ __device__ __forceinline__ void mma_commit_pair(uint32_t cluster_addr) {
                : "memory");
 }
 
+// ---------------- packed fp32 ----------------
+// two fp32 values in a register pair: {x, x}, and d = a * b + c per half (each half rounded as fmaf rounds it)
+__device__ __forceinline__ unsigned long long both(float x) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
 // ---------------- dependency counters ----------------
 __device__ __forceinline__ void red_release_add(unsigned *addr, unsigned v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(addr), "r"(v) : "memory");
