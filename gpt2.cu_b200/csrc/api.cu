@@ -190,13 +190,23 @@ static int run_gemm(GemmDesc &d, cudaStream_t st) {
   }
   GemmDesc dd = d;
   dd.out_bias = fused_bias;
-  // CTA pairs when the caller leaves the choice open (cta_pair = 0): 256 x 256 tiles stage a third less
-  // operand data per flop, which pays on the vocabulary-wide GEMMs (lm_head forward 1142 against 1225 us,
-  // backward_input 982 / 1011, backward_weight 982 / 1035) and not on the K = 768 layers, whose short tiles
-  // lose more to the pair's hand-shakes than they gain (attn_proj forward 47.6 against 42.4 us).
-  if (dd.opts.cta_pair == 0 && dd.opts.mode == GPT2L_MODE_TF32 && d.N >= 8192 && !dd.opts.xent_lse &&
-      ctx->max_pairs >= ctx->num_sms / 2)
-    dd.opts.cta_pair = 2;
+  // CTA pairs when the caller leaves the choice open (cta_pair = 0): 256 x 256 tiles stage a third less operand data per
+  // flop. What that saves grows with the k-blocks a pair works through; what it costs is a few microseconds of
+  // cluster launch and hand-shakes. TF32, 8192 rows (single CTAs / pairs, us): 768 -> 3072 forward 75.9 / 71.6,
+  // 3072 -> 768 78.4 / 73.0 (125 k-blocks a pair), 768 -> 768 28.9 / 31.0 (31); 768 -> 50304 1089 / 990. In 3xTF32 mode
+  // the operand split is a third less work per CTA as well: 328 / 248 and 350 / 254, 125 / 96; 2048 rows 768 -> 2304
+  // 70 / 58 (23); 1024 x 1024 x 1024 37 / 35, its weight gradient 39.7 / 41.2 (7).
+  if (dd.opts.cta_pair == 0 && !dd.opts.xent_lse && ctx->max_pairs >= ctx->num_sms / 2 && ctx->max_pairs > 0) {
+    const long long rows = d.kind == GPT2L_OP_BACKWARD_WEIGHT ? d.K : d.M;
+    const long long cols = d.kind == GPT2L_OP_BACKWARD_INPUT ? d.K : d.N;
+    const long long red = d.kind == GPT2L_OP_FORWARD ? d.K : d.kind == GPT2L_OP_BACKWARD_INPUT ? d.N : d.M;
+    const double kb_per_pair = (double)((rows + 255) / 256) * ((cols + 255) / 256) * ((red + BK - 1) / BK) / ctx->max_pairs;
+    // (a TF32 pair drains its tile with four warps per CTA, not eight: an epilogue that does more than store, GELU or an
+    // operand, costs what the main loop gains; the MLP's six calls at 8192 rows 595 us on single CTAs, 646 on pairs)
+    const bool plain = !dd.opts.aux_op && !(dd.opts.flags & GPT2L_EPI_GELU_DUAL);
+    if (dd.opts.mode == GPT2L_MODE_TF32X3 ? kb_per_pair >= 16.0 : (d.N >= 8192 || (plain && kb_per_pair >= 96.0)))
+      dd.opts.cta_pair = 2;
+  }
   GemmOp op;
   // Wide weight gradients (lm_head: N = 50304 against K = 768): the tensor core reads an MN-major A
   // operand about 20 % slower than a K-major one, and here A = in^T is tiny next to the GEMM. So

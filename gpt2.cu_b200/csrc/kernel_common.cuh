@@ -280,6 +280,27 @@ __device__ __forceinline__ float tf32_round(float x) {
 
 
 
+// 3xTF32: x = hi + lo with hi = x rounded to TF32, for N values of shared memory `step` float4 apart: all loads before the
+// first store, because a thread that waits out the latency of every value in turn (the compiler may not move a load past
+// a store it cannot tell apart) took 220 cycles per value.
+template <int N>
+__device__ __forceinline__ void split_hi_lo(float4 *hi, uint32_t lo_bytes, int first, int step, int end) {
+  float4 v[N];
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+    if (first + j * step < end) v[j] = hi[first + j * step];
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    if (first + j * step >= end) continue;
+    float4 h, l;
+    h.x = tf32_round(v[j].x); h.y = tf32_round(v[j].y); h.z = tf32_round(v[j].z); h.w = tf32_round(v[j].w);
+    l.x = v[j].x - h.x; l.y = v[j].y - h.y; l.z = v[j].z - h.z; l.w = v[j].w - h.w;
+    float4 *at = hi + first + j * step;
+    *at = h;
+    *reinterpret_cast<float4 *>(reinterpret_cast<uint8_t *>(at) + lo_bytes) = l;
+  }
+}
+
 // Epilogue store of one 32-row x 32-column chunk held as "thread = row, 32 consecutive columns"
 // (the tcgen05.ld 32x32b layout). Written straight from registers each thread would touch 32
 // different 128-byte lines per instruction; instead the chunk goes through a swizzled 4 KiB box in

@@ -126,7 +126,7 @@ __device__ __forceinline__ bool xform_tile(const GemmScalars *op, const Tile &tc
     // An MN-major B block is walked by (column group, k-row) so that the thread that sums a
     // column is also the one that rewrites it in 3xTF32 mode (no cross-thread hazard).
     // TMA zero-fills rows and columns outside the matrix, so no guards are needed.
-    const bool walk_b = op->b_mn && (X3 || cs_kb || xmode == 3);
+    const bool walk_b = op->b_mn && (cs_kb || xmode == 3);
     if (xmode == 2) {
       // row x of the A block: eight 16-byte chunks, chunk j at physical position j ^ (x & 7)
       uint8_t *arow = stage + x * 128;
@@ -183,19 +183,11 @@ __device__ __forceinline__ bool xform_tile(const GemmScalars *op, const Tile &tc
       }
     }
     if (X3) {
-      float4 *hi = reinterpret_cast<float4 *>(stage);
-      float4 *lo = reinterpret_cast<float4 *>(stage + rg.lo);
-      // what is left to split linearly: A (unless its rows were rewritten above) and a K-major B
+      // what is left to split linearly: A (unless its rows were rewritten above) and B (unless walked above)
       const int lin_lo = xmode == 2 ? (A_TILE_BYTES >> 4) : 0;
       const int lin_f4 = walk_b ? (A_TILE_BYTES >> 4) : stage_f4;
-      for (int i = lin_lo + x; i < lin_f4; i += NUM_XFORM_WARPS * 32) {
-        const float4 v = hi[i];
-        float4 h, l;
-        h.x = tf32_round(v.x); h.y = tf32_round(v.y); h.z = tf32_round(v.z); h.w = tf32_round(v.w);
-        l.x = v.x - h.x; l.y = v.y - h.y; l.z = v.z - h.z; l.w = v.w - h.w;
-        hi[i] = h;
-        lo[i] = l;
-      }
+      constexpr int T = NUM_XFORM_WARPS * 32;
+      for (int i = lin_lo + x; i < lin_f4; i += 8 * T) split_hi_lo<8>(reinterpret_cast<float4 *>(stage), rg.lo, i, T, lin_f4);
     }
     if (rewrites) fence_proxy_async_smem();
     __syncwarp();

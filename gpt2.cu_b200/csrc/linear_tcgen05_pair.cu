@@ -288,9 +288,8 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
         const GemmOp *maps;
         const GemmScalars *op = tile_at(t, cursor, tc, maps);
         const int bh = op->bn >> 1;
-        // the bias gradient belongs to tile row 0 (both CTAs of that pair: each sums its half of
-        // the columns)
-        const bool do_colsum = (op->colsum != nullptr) && tc.m_tile == 0 && op->b_mn;
+        // the bias gradient: every pair of tile rows takes its share of the k-blocks, each CTA its half of the columns
+        const bool do_colsum = (op->colsum != nullptr) && op->b_mn;
         const int groups = bh >> 2;
         const int parts = 128 / groups;
         const int rows_per_part = 32 / parts;
@@ -308,7 +307,7 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
           ok = __shfl_sync(0xffffffffu, okl, 0) != 0;
           if (!ok) break;
           uint8_t *stage = ring_ptr + s * STAGE_STRIDE;
-          const bool walk_b = op->b_mn && (X3 || do_colsum);
+          const bool walk_b = do_colsum && kb % op->tiles_dec == tc.m_tile;
           if (walk_b) {
             uint8_t *bchunk = stage + A_TILE_BYTES + chunk * 4096;
 #pragma unroll 4
@@ -327,17 +326,9 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
             }
           }
           if (X3) {
-            float4 *hi = reinterpret_cast<float4 *>(stage);
-            float4 *lo = reinterpret_cast<float4 *>(stage + LO_OFFSET);
             const int lin_f4 = walk_b ? (A_TILE_BYTES >> 4) : stage_f4;
-            for (int i = x; i < lin_f4; i += NUM_XFORM_WARPS * 32) {
-              const float4 v = hi[i];
-              float4 h, l;
-              h.x = tf32_round(v.x); h.y = tf32_round(v.y); h.z = tf32_round(v.z); h.w = tf32_round(v.w);
-              l.x = v.x - h.x; l.y = v.y - h.y; l.z = v.z - h.z; l.w = v.w - h.w;
-              hi[i] = h;
-              lo[i] = l;
-            }
+            constexpr int T = NUM_XFORM_WARPS * 32;
+            for (int i = x; i < lin_f4; i += 8 * T) split_hi_lo<8>(reinterpret_cast<float4 *>(stage), LO_OFFSET, i, T, lin_f4);
             fence_proxy_async_smem();
           }
           __syncwarp();
@@ -359,8 +350,7 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
             const float v[4] = {csum.x, csum.y, csum.z, csum.w};
             for (int j = 0; j < 4; ++j) {
               if (col + j < op->Nc) {
-                if (op->splits > 1) atomicAdd(op->colsum + col + j, v[j]);
-                else op->colsum[col + j] = v[j];
+                atomicAdd(op->colsum + col + j, v[j]);
               }
             }
           }
