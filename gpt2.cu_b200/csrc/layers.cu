@@ -714,6 +714,23 @@ __global__ void adamw_kernel(float *p, float *m, float *v, const float *g, long 
   }
 }
 
+// The gradients that a backward pass adds into, rather than writes: `head` floats (wpe) at g, then `pairs` layernorms of
+// 2C floats each, two a layer (at first and first + second, layers `layer` floats apart), the last one behind all layers.
+__global__ void __launch_bounds__(256)
+zero_accumulated_kernel(float *g, long long head, float *first, long long second, long long layer, long long last, int pairs,
+                        int two_c) {
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i < head) {
+    g[i] = 0.f;
+    return;
+  }
+  const long long j = i - head;
+  const int k = (int)(j / two_c), c = (int)(j % two_c);
+  if (k >= pairs) return;
+  const long long at = k == pairs - 1 ? last : (k >> 1) * layer + (k & 1) * second;
+  first[at + c] = 0.f;
+}
+
 // ------------------------------------------------------------------------------------
 // launchers
 // ------------------------------------------------------------------------------------
@@ -723,6 +740,12 @@ int embedding_forward(float *out, const int *tokens, const float *wte, const flo
                       cudaStream_t s) {
   const long long n = (long long)B * T * C;
   embedding_forward_kernel<<<cdiv(n, 256), 256, 0, s>>>(out, tokens, wte, wpe, B * T, T, C, Vp);
+  return LAUNCH_OK();
+}
+int zero_accumulated(float *g, long long head, float *first, long long second, long long layer, long long last, int pairs,
+                     int two_c, cudaStream_t s) {
+  zero_accumulated_kernel<<<cdiv(head + (long long)pairs * two_c, 256), 256, 0, s>>>(g, head, first, second, layer, last, pairs,
+                                                                                 two_c);
   return LAUNCH_OK();
 }
 int embedding_backward(float *g_wte, float *g_wpe, const float *g, const int *tokens, int B, int T, int C, int Vp,

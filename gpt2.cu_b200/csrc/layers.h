@@ -7,6 +7,10 @@ namespace g2l {
 
 int embedding_forward(float *out, const int *tokens, const float *wte, const float *wpe, int B, int T, int C, int Vp,
                       cudaStream_t s);
+// zeroes g[0 .. head) and `pairs` ranges of two_c floats, the k-th at first + (k / 2) * layer + (k % 2) * second, the last at
+// first + last
+int zero_accumulated(float *g, long long head, float *first, long long second, long long layer, long long last, int pairs,
+                     int two_c, cudaStream_t s);
 int embedding_backward(float *g_wte, float *g_wpe, const float *g, const int *tokens, int B, int T, int C, int Vp,
                        cudaStream_t s);
 int layernorm_forward(float *out, float *mean, float *rstd, const float *in, const float *w, const float *b, int M,

@@ -236,9 +236,12 @@ int gpt2_model_forward(gpt2_model *m, const int *tokens, const int *targets, gpt
   return GPT2L_OK;
 }
 
-// The backward pass in three parts, so that a data-parallel driver can hand each finished slice of
-// the gradient buffer to the all-reduce while the next part computes.
-int gpt2_model_backward_head(gpt2_model *m, gpt2l_stream_t stream) {
+}  // extern "C"
+
+// `whole`: every part of the backward pass follows, so only the gradients that kernels add into need to start at zero (wpe
+// and the layernorms; all others are overwritten, wte by the lm_head before the embedding adds to it). On its own the
+// head clears the whole buffer: the parts that are not run then leave zeros.
+static int backward_head(gpt2_model *m, bool whole, gpt2l_stream_t stream) {
   if (!m || !m->tokens) return GPT2L_ERR_BAD_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int B = m->B, T = m->T, C = m->cfg.n_embd, L = m->cfg.n_layer;
@@ -246,7 +249,14 @@ int gpt2_model_backward_head(gpt2_model *m, gpt2l_stream_t stream) {
   const int M = B * T;
   float *P = m->params, *G = m->grads;
   gpt2_linear_opts o = opts_for(m);
-  if (cudaMemsetAsync(G, 0, (size_t)m->n_params * sizeof(float), st) != cudaSuccess) return GPT2L_ERR_CUDA;
+  if (whole && L > 0) {  // (498 MB for GPT-2 small, 81 us, against 3 MB)
+    const LayerParams &p0 = m->lp[0];
+    const long long layer = L > 1 ? m->lp[1].ln1_w - p0.ln1_w : 0;
+    CK(zero_accumulated(G + m->off_wpe, (long long)m->cfg.n_positions * C, G + p0.ln1_w, p0.ln2_w - p0.ln1_w, layer,
+                        m->off_lnf_w - p0.ln1_w, 2 * L + 1, 2 * C, st));
+  } else if (cudaMemsetAsync(G, 0, (size_t)m->n_params * sizeof(float), st) != cudaSuccess) {
+    return GPT2L_ERR_CUDA;
+  }
   if (cudaMemsetAsync(m->dresid, 0, (size_t)M * C * sizeof(float), st) != cudaSuccess) return GPT2L_ERR_CUDA;
   // lm_head: the logits buffer holds dlogits since the forward pass — or, with the fused cross-entropy, still
   // the logits, which the two GEMMs turn into dlogits tile by tile as they read them
@@ -264,6 +274,12 @@ int gpt2_model_backward_head(gpt2_model *m, gpt2l_stream_t stream) {
                         m->lnf_mean, m->lnf_rstd, M, C, st));
   return GPT2L_OK;
 }
+
+extern "C" {
+
+// The backward pass in three parts, so that a data-parallel driver can hand each finished slice of
+// the gradient buffer to the all-reduce while the next part computes.
+int gpt2_model_backward_head(gpt2_model *m, gpt2l_stream_t stream) { return backward_head(m, false, stream); }
 
 int gpt2_model_backward_layer(gpt2_model *m, int l, gpt2l_stream_t stream) {
   if (!m || !m->tokens || l < 0 || l >= m->cfg.n_layer) return GPT2L_ERR_BAD_ARG;
@@ -306,7 +322,7 @@ int gpt2_model_backward_embedding(gpt2_model *m, gpt2l_stream_t stream) {
 
 int gpt2_model_backward(gpt2_model *m, gpt2l_stream_t stream) {
   if (!m) return GPT2L_ERR_BAD_ARG;
-  CK(gpt2_model_backward_head(m, stream));
+  CK(backward_head(m, true, stream));
   for (int l = m->cfg.n_layer - 1; l >= 0; --l) CK(gpt2_model_backward_layer(m, l, stream));
   return gpt2_model_backward_embedding(m, stream);
 }
