@@ -202,7 +202,8 @@ static int run_gemm(GemmDesc &d, cudaStream_t st) {
     const long long red = d.kind == GPT2L_OP_FORWARD ? d.K : d.kind == GPT2L_OP_BACKWARD_INPUT ? d.N : d.M;
     const double kb_per_pair = (double)((rows + 255) / 256) * ((cols + 255) / 256) * ((red + BK - 1) / BK) / ctx->max_pairs;
     // (a TF32 pair drains its tile with four warps per CTA, not eight: an epilogue that does more than store, GELU or an
-    // operand, costs what the main loop gains; the MLP's six calls at 8192 rows 595 us on single CTAs, 646 on pairs)
+    // operand, costs what the main loop gains; the MLP's six calls at 8192 rows: all on single CTAs 595 us, all on pairs
+    // 646, the three plain ones on pairs 577)
     const bool plain = !dd.opts.aux_op && !(dd.opts.flags & GPT2L_EPI_GELU_DUAL);
     if (dd.opts.mode == GPT2L_MODE_TF32X3 ? kb_per_pair >= 16.0 : (d.N >= 8192 || (plain && kb_per_pair >= 96.0)))
       dd.opts.cta_pair = 2;

@@ -827,14 +827,24 @@ static int encode_map_chunked(CUtensorMap *map, const float *base, uint64_t inne
 
 static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
-// Picks the tile width and the number of reduction splits: the pair that needs the fewest
-// (waves x per-tile work), where a tile's cost follows the bytes it pulls per k-block.
-static void choose_tiling(int Mc, int Nc, int kb_total, int num_sms, int forced_splits, bool pair, int *bn_out,
-                          int *splits_out) {
+// Picks the tile width and the number of reduction splits. Single CTAs in TF32 mode: by the time they should take, in
+// ns, from what was measured inside the kernel at 256 rows and over the GEMM set at 8192:
+//   - a k-block costs the loader and issuer 270 whatever the width (a 128 x 256 tile's MMAs 280); with the whole chip at
+//     work it waits for its operands, 330 / 370 / 450 for 64 / 128 / 256 columns;
+//   - draining a tile takes 2700 / 3500 / 5200; it hides behind the next tile's k-blocks, if any;
+//   - a split adds the zeroing of the output (a launch of its own) and its reduce-adds; the fixed-order combine passes
+//     through the workspace and costs several times as much. (fc forward at 256 rows, whose GELU store rules out
+//     reduce-adds: six splits of 256 columns 18.0 us, none of 64 columns 14.6; qkv forward 12.0 + 1.7 for the zeroing with
+//     eight splits, 8.6 with none.)
+// CTA pairs and 3xTF32, whose k-blocks cost several times more: the pair that needs the fewest (waves x per-tile work),
+// where a tile's cost follows the bytes it pulls per k-block.
+static void choose_tiling(int Mc, int Nc, int kb_total, int num_sms, int forced_splits, bool pair, bool by_time,
+                          bool fixed_order, int *bn_out, int *splits_out) {
   // scheduling units: SMs with 128-row tiles, or CTA pairs with 256-row tiles
   const int tile_rows = pair ? 2 * BM : BM;
   if (pair) num_sms = num_sms / 2 > 0 ? num_sms / 2 : 1;
   const int tiles_m = ceil_div(Mc, tile_rows);
+  const double out_bytes = 4.0 * Mc * Nc;
   double best = 1e300;
   int best_bn = 128, best_s = 1;
   const int cand[3] = {256, 128, 64};
@@ -843,6 +853,7 @@ static void choose_tiling(int Mc, int Nc, int kb_total, int num_sms, int forced_
     if (pair && bn < 128) continue;         // each CTA of a pair holds bn / 2 >= 64 columns of B
     if (bn > 64 && bn / 2 >= Nc) continue;  // tile twice as wide as the matrix
     const int tiles = tiles_m * ceil_div(Nc, bn);
+    const double drain = bn == 256 ? 5200.0 : (bn == 128 ? 3500.0 : 2700.0);
     const int smax = forced_splits > 0 ? forced_splits : (kb_total < 32 ? kb_total : 32);
     const int smin = forced_splits > 0 ? forced_splits : 1;
     for (int s = smin; s <= smax; ++s) {
@@ -850,10 +861,18 @@ static void choose_tiling(int Mc, int Nc, int kb_total, int num_sms, int forced_
       const int per = ceil_div(kb_total, s);
       if (forced_splits == 0 && s > 1 && (s - 1) * per >= kb_total) continue;  // an empty split
       const double waves = (double)ceil_div(tiles * s, num_sms);
-      // + 6 k-blocks of fixed per-tile overhead (pipeline fill, epilogue); splits pay an extra pass over the
-      // output (two k-blocks' worth since the partials go out as reduce-adds of the copy engine; measured on the
-      // qkv weight gradient at M = 16384: 8 splits 153 us, 5 splits 163 us)
-      const double cost = waves * (per + 6.0 + (s > 1 ? 2.0 : 0.0)) * (double)(tile_rows + bn);
+      double cost;
+      if (by_time) {
+        const int units = tiles * s < num_sms ? tiles * s : num_sms;
+        const double loaded = 206.0 + (double)(A_TILE_BYTES + bn * BK * 4) * units / 29600.0;
+        const double body = per * (loaded > 270.0 ? loaded : 270.0);
+        cost = (waves - 1.0) * (body > drain ? body : drain) + body + drain;
+        if (s > 1) cost += fixed_order ? 4000.0 + out_bytes * s / 3000.0 : 1500.0 + out_bytes * s / 8000.0;
+      } else {
+        // + 6 k-blocks of fixed per-tile overhead (pipeline fill, epilogue); splits pay an extra pass over the
+        // output (two k-blocks' worth since the partials go out as reduce-adds of the copy engine)
+        cost = waves * (per + 6.0 + (s > 1 ? 2.0 : 0.0)) * (double)(tile_rows + bn);
+      }
       if (cost < best - 1e-9) {
         best = cost;
         best_bn = bn;
@@ -929,7 +948,8 @@ int plan_op(const GemmDesc &d, int num_sms, GemmOp *op) {
   // CTA pairs (256-row tiles, B split between the two CTAs) cut operand traffic per flop by a third; whether
   // that pays depends on the shape, so the choice is the caller's (the public entry points pick for cta_pair = 0)
   op->pair = (d.opts.cta_pair == 2) ? 1 : 0;
-  choose_tiling(op->Mc, op->Nc, op->kb_total, num_sms > 0 ? num_sms : 148, forced, op->pair != 0, &bn, &splits);
+  choose_tiling(op->Mc, op->Nc, op->kb_total, num_sms > 0 ? num_sms : 148, forced, op->pair != 0,
+                !op->pair && op->mode == GPT2L_MODE_TF32, d.opts.deterministic != 0 || op->C2 != nullptr, &bn, &splits);
   op->bn = bn;
   op->kb_per_split = ceil_div(op->kb_total, splits);
   op->splits = ceil_div(op->kb_total, op->kb_per_split);  // no empty trailing split
