@@ -15,8 +15,8 @@
 // and write it back over the scores (tcgen05.st) -> accumulate MMAs that take that tile as their A
 // operand straight from TMEM", so they share one skeleton; P and dS never touch shared memory, which
 // saves the 32 KiB tile per step, its stores and the proxy fence they would need, and leaves the room
-// for double-buffered operand stages (measured: a 128 x 64 x 8 TF32 MMA costs about 75 ns from one CTA
-// wherever its A operand lives; two resident CTAs overlap to about 38 ns each): warp 0 loads operands with TMA straight out of qkv[B*T][3C] / dout[B*T][C] (batched
+// for double-buffered operand stages (a 128 x 64 x 8 TF32 MMA costs 49 cycles
+// when MMAs are queued, wherever its A operand lives): warp 0 loads operands with TMA straight out of qkv[B*T][3C] / dout[B*T][C] (batched
 // tensor maps, nothing is copied or transposed), warp 1 issues the MMAs (BWD_KV: warp 1 the score MMAs,
 // warp 2 the accumulate MMAs), the remaining 4 (BWD_KV: 8) warps do the row work.
 // In FWD and BWD_KV score buffers rotate through three TMEM slots (the score MMAs of block t+1 run while
@@ -86,9 +86,9 @@ int launch(const FlashMaps &maps, const FlashArgs &args, cudaStream_t st) {
     attr_set = true;
   }
   const int grid = args.B * args.NH * (args.T / FROWS);
-  attn_flash_kernel<MODE><<<grid, Cfg<MODE>::THREADS, Cfg<MODE>::SMEM, st>>>(maps, args);
+  const cudaError_t e = launch_pdl(attn_flash_kernel<MODE>, grid, Cfg<MODE>::THREADS, Cfg<MODE>::SMEM, st, maps, args);
   count_launch();
-  return cudaGetLastError() == cudaSuccess ? GPT2L_OK : GPT2L_ERR_CUDA;
+  return e == cudaSuccess ? GPT2L_OK : GPT2L_ERR_CUDA;
 }
 
 }  // namespace

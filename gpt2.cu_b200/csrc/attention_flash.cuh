@@ -587,6 +587,8 @@ attn_flash_kernel(const __grid_constant__ FlashMaps maps, const FlashArgs a) {
   tc_fence_after();
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(&ctrl->tmem_base);
 
+  pdl_trigger();
+  pdl_wait();
   attn_tile_body<MODE>(maps, a, base_ptr, base, ctrl, tmem, warp, lane, rb, bh, 0u, 0u);
 
   // =============================== teardown ===============================

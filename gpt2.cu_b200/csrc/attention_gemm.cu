@@ -18,6 +18,7 @@
 
 #include "layers.h"
 #include "linear_internal.h"
+#include "ptx_sm100.cuh"
 
 namespace g2l {
 
@@ -27,6 +28,8 @@ constexpr int AHS = 64;
 // the row's 128-column block (what the P.V and P^T.dO reductions read past the diagonal).
 __global__ void __launch_bounds__(256)
 attn_softmax_kernel(float *S, int T, long long rows, float scale) {
+  ptx::pdl_trigger();
+  ptx::pdl_wait();
   const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (r >= rows) return;
   const int lane = threadIdx.x & 31;
@@ -48,6 +51,8 @@ attn_softmax_kernel(float *S, int T, long long rows, float scale) {
 // T x T tensors): one warp per (b, i, h), two of the 64 head values per lane.
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(float *delta, const float *dout, const float *out, int T, int C, int NH, long long rows) {
+  ptx::pdl_trigger();
+  ptx::pdl_wait();
   const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);  // (b*T + i)*NH + h
   if (r >= rows) return;
   const int lane = threadIdx.x & 31;
@@ -63,9 +68,9 @@ attn_delta_kernel(float *delta, const float *dout, const float *out, int T, int 
 // delta[B][NH][T] = rowsum(dout o out) per head
 int attention_row_dot(float *delta, const float *dout, const float *out, int B, int T, int C, int NH, cudaStream_t st) {
   const long long rows = (long long)B * NH * T;
-  attn_delta_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(delta, dout, out, T, C, NH, rows);
+  const cudaError_t e = launch_pdl(attn_delta_kernel, (unsigned)((rows + 7) / 8), 256, 0, st, delta, dout, out, T, C, NH, rows);
   count_launch();
-  return cudaGetLastError() == cudaSuccess ? GPT2L_OK : GPT2L_ERR_CUDA;
+  return e == cudaSuccess ? GPT2L_OK : GPT2L_ERR_CUDA;
 }
 
 static int run(DeviceCtx *ctx, const BatchedDesc &d, cudaStream_t st) {
@@ -96,9 +101,9 @@ int attention_forward_gemm(float *out, float *P, const float *qkv, int B, int T,
   d.causal = 1; d.mode = mode;
   if ((err = run(ctx, d, st))) return err;
   const long long rows = (long long)B * NH * T;
-  attn_softmax_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(P, T, rows, 0.125f);
+  const cudaError_t le = launch_pdl(attn_softmax_kernel, (unsigned)((rows + 7) / 8), 256, 0, st, P, T, rows, 0.125f);
   count_launch();
-  if (cudaGetLastError() != cudaSuccess) return GPT2L_ERR_CUDA;
+  if (le != cudaSuccess) return GPT2L_ERR_CUDA;
   // O = P V
   d.Mc = T; d.Nc = AHS; d.Kc = T; d.a_mn = 0; d.b_mn = 1;
   d.a = P; d.b = qkv + 2 * C; d.c = out;

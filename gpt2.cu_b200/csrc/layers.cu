@@ -24,6 +24,8 @@ static inline int cdiv(long long a, int b) { return (int)((a + b - 1) / b); }
 // ------------------------------------------------------------------------------------
 __global__ void embedding_forward_kernel(float *out, const int *tokens, const float *wte, const float *wpe, int M,
                                          int T, int C, int Vp) {
+  ptx::pdl_trigger();
+  ptx::pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long long)M * C) return;
   const int m = (int)(i / C), c = (int)(i % C);
@@ -35,6 +37,8 @@ __global__ void embedding_forward_kernel(float *out, const int *tokens, const fl
 // embedding.cu:93, which does not match its own forward; the PyTorch model is the semantics kept.)
 __global__ void embedding_backward_kernel(float *g_wte, float *g_wpe, const float *g, const int *tokens, int M, int T,
                                           int C, int Vp) {
+  ptx::pdl_trigger();
+  ptx::pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long long)M * C) return;
   const int m = (int)(i / C), c = (int)(i % C);
@@ -56,6 +60,8 @@ __device__ __forceinline__ float warp_sum(float v) {
 __global__ void __launch_bounds__(256)
 layernorm_forward_kernel(float *out, float *mean, float *rstd, const float *in, const float *w, const float *b,
                          int M, int C) {
+  ptx::pdl_trigger();
+  ptx::pdl_wait();
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= M) return;
@@ -76,6 +82,8 @@ template <int K4>  // C <= 128 * K4, C a multiple of 4
 __global__ void __launch_bounds__(256)
 layernorm_forward_vec_kernel(float *out, float *mean, float *rstd, const float *in, const float *w, const float *b,
                              int M, int C) {
+  ptx::pdl_trigger();
+  ptx::pdl_wait();
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= M) return;
@@ -123,6 +131,8 @@ template <int K4>  // float4 columns per lane: C <= 128 * K4 (C is a multiple of
 __global__ void __launch_bounds__(256, (K4 <= 6 ? 2 : 1))
 layernorm_backward_kernel(float *g_in, float *g_w, float *g_b, const float *g_out, const float *in, const float *w,
                           const float *mean, const float *rstd, int M, int C, int rows_per_block) {
+  ptx::pdl_trigger();
+  ptx::pdl_wait();
   extern __shared__ __align__(16) float sm[];  // [4][C]: column sums of four warps
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   float4 aw[K4], ab[K4];
@@ -375,6 +385,8 @@ softmax_xent_large_kernel(float *logits, float *losses, const int *targets, int 
 // ------------------------------------------------------------------------------------
 __global__ void xent_combine_kernel(float *lse, float *losses, const float2 *stats, int stride, const float *logits,
                                     long long ld, const int *targets, int M) {
+  ptx::pdl_trigger();
+  ptx::pdl_wait();
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= M) return;
@@ -404,6 +416,8 @@ __global__ void xent_combine_kernel(float *lse, float *losses, const float2 *sta
 // sums are known already, so nothing is reduced here). A block per row.
 __global__ void __launch_bounds__(512)
 xent_grad_inplace_kernel(float *logits, const float *lse, const int *targets, int V, int Vp, float scale) {
+  ptx::pdl_trigger();
+  ptx::pdl_wait();
   float *row = logits + (long long)blockIdx.x * Vp;
   const float l2 = lse[blockIdx.x];
   const int tgt = targets[blockIdx.x];
@@ -692,6 +706,8 @@ __device__ __forceinline__ void adamw_one(float &p, float &m, float &v, float gi
 // tail (a range of the flat buffer may start anywhere); every element sees the same arithmetic.
 __global__ void adamw_kernel(float *p, float *m, float *v, const float *g, long long n, long long head, long long n4,
                              float lr, float b1, float b2, float eps, float wd, float bc1, float bc2) {
+  ptx::pdl_trigger();
+  ptx::pdl_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n4) {
     const long long o = head + 4 * i;
@@ -719,6 +735,8 @@ __global__ void adamw_kernel(float *p, float *m, float *v, const float *g, long 
 __global__ void __launch_bounds__(256)
 zero_accumulated_kernel(float *g, long long head, float *first, long long second, long long layer, long long last, int pairs,
                         int two_c) {
+  ptx::pdl_trigger();
+  ptx::pdl_wait();
   const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
   if (i < head) {
     g[i] = 0.f;
@@ -735,29 +753,34 @@ zero_accumulated_kernel(float *g, long long head, float *first, long long second
 // launchers
 // ------------------------------------------------------------------------------------
 #define LAUNCH_OK() (count_launch(), cudaGetLastError() == cudaSuccess ? GPT2L_OK : GPT2L_ERR_CUDA)
+#define PDL_OK() (count_launch(), le == cudaSuccess ? GPT2L_OK : GPT2L_ERR_CUDA)
 
 int embedding_forward(float *out, const int *tokens, const float *wte, const float *wpe, int B, int T, int C, int Vp,
                       cudaStream_t s) {
+  cudaError_t le;
   const long long n = (long long)B * T * C;
-  embedding_forward_kernel<<<cdiv(n, 256), 256, 0, s>>>(out, tokens, wte, wpe, B * T, T, C, Vp);
-  return LAUNCH_OK();
+  le = launch_pdl(embedding_forward_kernel, cdiv(n, 256), 256, 0, s, out, tokens, wte, wpe, B * T, T, C, Vp);
+  return PDL_OK();
 }
 int zero_accumulated(float *g, long long head, float *first, long long second, long long layer, long long last, int pairs,
                      int two_c, cudaStream_t s) {
-  zero_accumulated_kernel<<<cdiv(head + (long long)pairs * two_c, 256), 256, 0, s>>>(g, head, first, second, layer, last, pairs,
+  cudaError_t le;
+  le = launch_pdl(zero_accumulated_kernel, cdiv(head + (long long)pairs * two_c, 256), 256, 0, s, g, head, first, second, layer, last, pairs,
                                                                                  two_c);
-  return LAUNCH_OK();
+  return PDL_OK();
 }
 int embedding_backward(float *g_wte, float *g_wpe, const float *g, const int *tokens, int B, int T, int C, int Vp,
                        cudaStream_t s) {
+  cudaError_t le;
   const long long n = (long long)B * T * C;
-  embedding_backward_kernel<<<cdiv(n, 256), 256, 0, s>>>(g_wte, g_wpe, g, tokens, B * T, T, C, Vp);
-  return LAUNCH_OK();
+  le = launch_pdl(embedding_backward_kernel, cdiv(n, 256), 256, 0, s, g_wte, g_wpe, g, tokens, B * T, T, C, Vp);
+  return PDL_OK();
 }
 int layernorm_forward(float *out, float *mean, float *rstd, const float *in, const float *w, const float *b, int M,
                       int C, cudaStream_t s) {
-#define LN_FWD(K4) layernorm_forward_vec_kernel<K4><<<cdiv(M, 8), 256, 0, s>>>(out, mean, rstd, in, w, b, M, C)
-  if (C & 3) layernorm_forward_kernel<<<cdiv(M, 8), 256, 0, s>>>(out, mean, rstd, in, w, b, M, C);
+  cudaError_t le;
+#define LN_FWD(K4) le = launch_pdl(layernorm_forward_vec_kernel<K4>, cdiv(M, 8), 256, 0, s, out, mean, rstd, in, w, b, M, C)
+  if (C & 3) le = launch_pdl(layernorm_forward_kernel, cdiv(M, 8), 256, 0, s, out, mean, rstd, in, w, b, M, C);
   else if (C <= 128) LN_FWD(1);
   else if (C <= 256) LN_FWD(2);
   else if (C <= 512) LN_FWD(4);
@@ -765,12 +788,13 @@ int layernorm_forward(float *out, float *mean, float *rstd, const float *in, con
   else if (C <= 1024) LN_FWD(8);
   else if (C <= 1280) LN_FWD(10);
   else if (C <= 2048) LN_FWD(16);
-  else layernorm_forward_kernel<<<cdiv(M, 8), 256, 0, s>>>(out, mean, rstd, in, w, b, M, C);
+  else le = launch_pdl(layernorm_forward_kernel, cdiv(M, 8), 256, 0, s, out, mean, rstd, in, w, b, M, C);
 #undef LN_FWD
-  return LAUNCH_OK();
+  return PDL_OK();
 }
 int layernorm_backward(float *g_in, float *g_w, float *g_b, const float *g_out, const float *in, const float *w,
                        const float *mean, const float *rstd, int M, int C, cudaStream_t s) {
+  cudaError_t le;
   // one block per resident slot (two per SM) where there are rows enough: every block then ends at about
   // the same time, and the column sums meet in global memory only ~300 times; a row per warp where there are not
   static const int slots = [] {
@@ -784,7 +808,7 @@ int layernorm_backward(float *g_in, float *g_w, float *g_b, const float *g_out, 
   const int blocks = cdiv(M, rows_per_block);
   const size_t smem = 4 * (size_t)C * sizeof(float);
   if (C & 3) return GPT2L_ERR_BAD_ARG;
-#define LN_BWD(K4) layernorm_backward_kernel<K4><<<blocks, 256, smem, s>>>(g_in, g_w, g_b, g_out, in, w, mean, rstd, M, C, rows_per_block)
+#define LN_BWD(K4) le = launch_pdl(layernorm_backward_kernel<K4>, blocks, 256, smem, s, g_in, g_w, g_b, g_out, in, w, mean, rstd, M, C, rows_per_block)
   if (C <= 128) LN_BWD(1);
   else if (C <= 256) LN_BWD(2);
   else if (C <= 512) LN_BWD(4);
@@ -794,7 +818,7 @@ int layernorm_backward(float *g_in, float *g_w, float *g_b, const float *g_out, 
   else if (C <= 2048) LN_BWD(16);
   else return GPT2L_ERR_TOO_LARGE;
 #undef LN_BWD
-  return LAUNCH_OK();
+  return PDL_OK();
 }
 int add_forward(float *out, const float *a, const float *b, long long n, cudaStream_t s) {
   add_kernel<<<cdiv((n + 3) / 4, 256), 256, 0, s>>>(out, a, b, n);
@@ -822,14 +846,16 @@ int softmax_xent(float *logits, float *losses, const int *targets, int M, int V,
 }
 int launch_xent_combine(float *lse, float *losses, const float *stats, int stride, const float *logits, long long ld,
                         const int *targets, int M, cudaStream_t s) {
-  xent_combine_kernel<<<cdiv(M, 8), 256, 0, s>>>(lse, losses, reinterpret_cast<const float2 *>(stats), stride, logits, ld,
+  cudaError_t le;
+  le = launch_pdl(xent_combine_kernel, cdiv(M, 8), 256, 0, s, lse, losses, reinterpret_cast<const float2 *>(stats), stride, logits, ld,
                                                   targets, M);
-  return LAUNCH_OK();
+  return PDL_OK();
 }
 int xent_grad_inplace(float *logits, const float *lse, const int *targets, int M, int V, int Vp, cudaStream_t s) {
+  cudaError_t le;
   if (Vp & 3) return GPT2L_ERR_BAD_ARG;
-  xent_grad_inplace_kernel<<<M, 512, 0, s>>>(logits, lse, targets, V, Vp, 1.f / (float)M);
-  return LAUNCH_OK();
+  le = launch_pdl(xent_grad_inplace_kernel, M, 512, 0, s, logits, lse, targets, V, Vp, 1.f / (float)M);
+  return PDL_OK();
 }
 int attention_forward(float *out, float *lse, const float *qkv, int B, int T, int C, int NH, cudaStream_t s) {
   if (C != NH * HS) return GPT2L_ERR_BAD_ARG;
@@ -857,14 +883,15 @@ int attention_backward(float *dqkv, float *delta, const float *dout, const float
 }
 int adamw_update(float *p, float *m, float *v, const float *g, long long n, float lr, float b1, float b2, float eps,
                  float wd, int t, cudaStream_t s) {
+  cudaError_t le;
   const float bc1 = 1.f - powf(b1, (float)t), bc2 = 1.f - powf(b2, (float)t);
   // all four buffers are offset alike from 256-byte aligned allocations, so p decides the alignment
   long long head = (long long)((16 - (reinterpret_cast<uintptr_t>(p) & 15)) & 15) / 4;
   if (head > n) head = n;
   const long long n4 = (n - head) / 4;
   const long long extra = n - 4 * n4;  // head + tail, at most 6
-  adamw_kernel<<<cdiv(n4 + extra, 256), 256, 0, s>>>(p, m, v, g, n, head, n4, lr, b1, b2, eps, wd, bc1, bc2);
-  return LAUNCH_OK();
+  le = launch_pdl(adamw_kernel, cdiv(n4 + extra, 256), 256, 0, s, p, m, v, g, n, head, n4, lr, b1, b2, eps, wd, bc1, bc2);
+  return PDL_OK();
 }
 
 }  // namespace g2l

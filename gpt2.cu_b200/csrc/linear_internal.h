@@ -323,6 +323,25 @@ int launch_list(DeviceCtx *ctx, const GemmOp *d_ops, int n_ops, int total_tiles,
 int set_kernel_attributes();
 void count_launch(int n = 1);
 
+// Launch that may overlap the tail of the kernel before it in the stream (see pdl_wait in ptx_sm100.cuh, which the
+// kernel must execute): launch latency, barrier set-up and tensor-memory allocation then come off the critical path.
+template <class... P, class... A>
+cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return e;
+}
+
 // --- attention_flash.cu ---
 // tensor maps of the fused attention over qkv[B*T][3C] and dout[B*T][C] (dout may be null: forward)
 int attention_flash_build_maps(FlashMaps *maps, const float *qkv, const float *dout, int B, int T, int C, int NH);

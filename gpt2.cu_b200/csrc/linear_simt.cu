@@ -244,6 +244,8 @@ gpt2_linear_colsum_kernel(float *__restrict__ out, const float *__restrict__ x, 
 // dst[c][r] = src[r][c] for src[rows][cols]; 32 x 32 tiles through shared memory, both sides coalesced.
 __global__ void __launch_bounds__(256)
 gpt2_linear_transpose_kernel(float *__restrict__ dst, const float *__restrict__ src, int rows, int cols) {
+  ptx::pdl_trigger();
+  ptx::pdl_wait();
   __shared__ float tile[32][33];
   const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
   const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
@@ -260,9 +262,9 @@ gpt2_linear_transpose_kernel(float *__restrict__ dst, const float *__restrict__ 
 
 int launch_transpose(float *dst, const float *src, int rows, int cols, cudaStream_t stream) {
   dim3 grid((cols + 31) / 32, (rows + 31) / 32);
-  gpt2_linear_transpose_kernel<<<grid, 256, 0, stream>>>(dst, src, rows, cols);
+  const cudaError_t e = launch_pdl(gpt2_linear_transpose_kernel, grid, 256, 0, stream, dst, src, rows, cols);
   count_launch();
-  return cudaGetLastError() == cudaSuccess ? GPT2L_OK : GPT2L_ERR_CUDA;
+  return e == cudaSuccess ? GPT2L_OK : GPT2L_ERR_CUDA;
 }
 
 namespace {

@@ -554,6 +554,10 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(&ctrl->tmem_base);
   const Ring<X3, MEGA> rg(MEGA ? 0 : staged->bn);
+  if (!MEGA) {
+    pdl_trigger();
+    pdl_wait();
+  }
 
   if (warp == 0) {
     // =============================== TMA producer ===============================
@@ -1147,12 +1151,13 @@ int launch_single(DeviceCtx *ctx, GemmOp &op, cudaStream_t stream) {
     return pair_launch(&op, p, pairs, op.mode == GPT2L_MODE_TF32X3, stream);
   }
   const int grid = op.n_tiles < ctx->num_sms ? op.n_tiles : ctx->num_sms;
+  cudaError_t e;
   if (op.mode == GPT2L_MODE_TF32X3)
-    gpt2_linear_tcgen05_kernel<true, false><<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(op, p);
+    e = launch_pdl(gpt2_linear_tcgen05_kernel<true, false>, grid, NUM_THREADS, SMEM_BYTES, stream, op, p);
   else
-    gpt2_linear_tcgen05_kernel<false, false><<<grid, NUM_THREADS, SMEM_BYTES, stream>>>(op, p);
+    e = launch_pdl(gpt2_linear_tcgen05_kernel<false, false>, grid, NUM_THREADS, SMEM_BYTES, stream, op, p);
   count_launch();
-  return cudaGetLastError() == cudaSuccess ? GPT2L_OK : GPT2L_ERR_CUDA;
+  return e == cudaSuccess ? GPT2L_OK : GPT2L_ERR_CUDA;
 }
 
 // One launch over a device array of ops. GEMM-only lists on CTA pairs keep the pair kernel; everything

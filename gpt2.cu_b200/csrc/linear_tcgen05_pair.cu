@@ -115,6 +115,8 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
   cluster_sync_all();  // the peer's barriers exist before anyone arrives on them
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(&ctrl->tmem_base);
+  pdl_trigger();
+  pdl_wait();
 
   if (warp == 0) {
     // =============================== TMA producer (both CTAs) ===============================
@@ -407,7 +409,7 @@ int pair_set_kernel_attributes() {
   return e == cudaSuccess ? GPT2L_OK : GPT2L_ERR_CUDA;
 }
 
-static void fill_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr, int n_pairs, cudaStream_t stream) {
+static void fill_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr, int n_pairs, bool overlap, cudaStream_t stream) {
   memset(cfg, 0, sizeof(*cfg));
   cfg->gridDim = dim3(2 * n_pairs, 1, 1);
   cfg->blockDim = dim3(NUM_THREADS, 1, 1);
@@ -417,14 +419,16 @@ static void fill_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr, int 
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // (see launch_pdl)
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg->attrs = attr;
-  cfg->numAttrs = 1;
+  cfg->numAttrs = overlap ? 2 : 1;
 }
 
 int pair_max_pairs(int num_sms) {
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute attr[1];
-  fill_config(&cfg, attr, num_sms / 2, nullptr);
+  cudaLaunchAttribute attr[2];
+  fill_config(&cfg, attr, num_sms / 2, false, nullptr);
   int clusters = 0;
   if (cudaOccupancyMaxActiveClusters(&clusters, gpt2_linear_tcgen05_pair_kernel<false>, &cfg) != cudaSuccess) {
     (void)cudaGetLastError();
@@ -437,8 +441,8 @@ int pair_max_pairs(int num_sms) {
 int pair_launch(const GemmOp *op_by_value, const LaunchParams &p, int n_pairs, bool x3, cudaStream_t stream) {
   static GemmOp dummy;
   cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute attr[1];
-  fill_config(&cfg, attr, n_pairs, stream);
+  cudaLaunchAttribute attr[2];
+  fill_config(&cfg, attr, n_pairs, op_by_value != nullptr, stream);
   const GemmOp &op = op_by_value ? *op_by_value : dummy;
   cudaError_t e;
   if (x3) e = cudaLaunchKernelEx(&cfg, gpt2_linear_tcgen05_pair_kernel<true>, op, p);

@@ -304,6 +304,14 @@ __device__ __forceinline__ void mma_commit_pair(uint32_t cluster_addr) {
                : "memory");
 }
 
+// ---------------- programmatic dependent launch ----------------
+// A kernel launched with launch_pdl may start while the kernel before it in the stream still runs. trigger: the next one
+// may start once every block of this grid has said so (or ended); wait: everything the kernels before this one did
+// is complete and visible. No kernel touches global memory that another kernel writes, or writes any, before its wait, so
+// each kernel's end implies the end of all before it.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------- packed fp32 ----------------
 // two fp32 values in a register pair: {x, x}, and d = a * b + c per half (each half rounded as fmaf rounds it)
 __device__ __forceinline__ unsigned long long both(float x) {
