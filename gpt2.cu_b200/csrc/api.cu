@@ -238,21 +238,19 @@ static int run_gemm(GemmDesc &d, cudaStream_t st) {
     op.colsum_spread = fused_bias ? 1 : 0;
     op.cs_src = d.b;
   }
-  if (op.splits > 1) {
-    if (op.atomic_out) {
-      if (cudaMemsetAsync(op.C, 0, (size_t)op.Mc * op.Nc * sizeof(float), st) != cudaSuccess) return GPT2L_ERR_CUDA;
-    } else {
-      std::lock_guard<std::mutex> lk(g_mu);
-      if ((size_t)op.tiles_m * op.tiles_n * 4 > ctx->ws_sem_count) return GPT2L_ERR_TOO_LARGE;
-      err = ensure_bytes(&ctx->ws, &ctx->ws_bytes, op_workspace_bytes(op));
-      if (err) return err;
-      op.ws = ctx->ws;
-      op.ws_sem = ctx->ws_sem;
-    }
-    if (op.colsum && cudaMemsetAsync(op.colsum, 0, (size_t)op.Nc * sizeof(float), st) != cudaSuccess)
-      return GPT2L_ERR_CUDA;
-  } else if (op.colsum && op.colsum_spread) {
-    if (cudaMemsetAsync(op.colsum, 0, (size_t)op.Nc * sizeof(float), st) != cudaSuccess) return GPT2L_ERR_CUDA;
+  if (op.splits > 1 && !op.atomic_out) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if ((size_t)op.tiles_m * op.tiles_n * 4 > ctx->ws_sem_count) return GPT2L_ERR_TOO_LARGE;
+    err = ensure_bytes(&ctx->ws, &ctx->ws_bytes, op_workspace_bytes(op));
+    if (err) return err;
+    op.ws = ctx->ws;
+    op.ws_sem = ctx->ws_sem;
+  }
+  // (Nc is a multiple of four and C 16-byte aligned: tma_eligible)
+  const bool zero_c = op.splits > 1 && op.atomic_out, zero_cs = op.colsum && (op.splits > 1 || op.colsum_spread);
+  if (zero_c || zero_cs) {
+    err = launch_zero(op.C, zero_c ? (long long)op.Mc * op.Nc : 0, op.colsum, zero_cs ? op.Nc : 0, st);
+    if (err) return err;
   }
   err = launch_single(ctx, op, st);
   if (err) return err;

@@ -349,6 +349,8 @@ int attention_flash_build_maps(FlashMaps *maps, const float *qkv, const float *d
 // --- linear_simt.cu ---
 int launch_simt(const GemmDesc &d, cudaStream_t stream);
 int launch_colsum(float *out, const float *x, int rows, int cols, cudaStream_t stream);
+// zeroes a[0 .. n) (16-byte aligned, n a multiple of four; may be empty) and b[0 .. nb)
+int launch_zero(float *a, long long n, float *b, int nb, cudaStream_t stream);
 int launch_transpose(float *dst, const float *src, int rows, int cols, cudaStream_t stream);
 // floats of statistics a forward GEMM with xent_stats leaves: rows * stride(op) * 2
 size_t xent_stats_floats(const GemmOp &op);

@@ -260,6 +260,24 @@ gpt2_linear_transpose_kernel(float *__restrict__ dst, const float *__restrict__ 
   }
 }
 
+// What a split or a bias gradient adds into: a[0 .. 4 n4) and b[0 .. nb). One launch that may overlap the kernel before it
+// (a memset may not, and stood between the launches of a chain twice per call).
+__global__ void __launch_bounds__(256)
+gpt2_linear_zero_kernel(float4 *a, long long n4, float *b, int nb) {
+  ptx::pdl_trigger();
+  ptx::pdl_wait();
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i < n4) a[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  else if (i - n4 < nb) b[i - n4] = 0.f;
+}
+
+int launch_zero(float *a, long long n, float *b, int nb, cudaStream_t stream) {
+  const cudaError_t e = launch_pdl(gpt2_linear_zero_kernel, dim3((unsigned)((n / 4 + nb + 255) / 256)), 256, 0, stream,
+                                   reinterpret_cast<float4 *>(a), n / 4, b, nb);
+  count_launch();
+  return e == cudaSuccess ? GPT2L_OK : GPT2L_ERR_CUDA;
+}
+
 int launch_transpose(float *dst, const float *src, int rows, int cols, cudaStream_t stream) {
   dim3 grid((cols + 31) / 32, (rows + 31) / 32);
   const cudaError_t e = launch_pdl(gpt2_linear_transpose_kernel, grid, 256, 0, stream, dst, src, rows, cols);
