@@ -190,24 +190,7 @@ static int run_gemm(GemmDesc &d, cudaStream_t st) {
   }
   GemmDesc dd = d;
   dd.out_bias = fused_bias;
-  // CTA pairs when the caller leaves the choice open (cta_pair = 0): 256 x 256 tiles stage a third less operand data per
-  // flop. What that saves grows with the k-blocks a pair works through; what it costs is a few microseconds of
-  // cluster launch and hand-shakes. TF32, 8192 rows (single CTAs / pairs, us): 768 -> 3072 forward 75.9 / 71.6,
-  // 3072 -> 768 78.4 / 73.0 (125 k-blocks a pair), 768 -> 768 28.9 / 31.0 (31); 768 -> 50304 1089 / 990. In 3xTF32 mode
-  // the operand split is a third less work per CTA as well: 328 / 248 and 350 / 254, 125 / 96; 2048 rows 768 -> 2304
-  // 70 / 58 (23); 1024 x 1024 x 1024 37 / 35, its weight gradient 39.7 / 41.2 (7).
-  if (dd.opts.cta_pair == 0 && !dd.opts.xent_lse && ctx->max_pairs >= ctx->num_sms / 2 && ctx->max_pairs > 0) {
-    const long long rows = d.kind == GPT2L_OP_BACKWARD_WEIGHT ? d.K : d.M;
-    const long long cols = d.kind == GPT2L_OP_BACKWARD_INPUT ? d.K : d.N;
-    const long long red = d.kind == GPT2L_OP_FORWARD ? d.K : d.kind == GPT2L_OP_BACKWARD_INPUT ? d.N : d.M;
-    const double kb_per_pair = (double)((rows + 255) / 256) * ((cols + 255) / 256) * ((red + BK - 1) / BK) / ctx->max_pairs;
-    // (a TF32 pair drains its tile with four warps per CTA, not eight: an epilogue that does more than store, GELU or an
-    // operand, costs what the main loop gains; the MLP's six calls at 8192 rows: all on single CTAs 595 us, all on pairs
-    // 646, the three plain ones on pairs 577)
-    const bool plain = !dd.opts.aux_op && !(dd.opts.flags & GPT2L_EPI_GELU_DUAL);
-    if (dd.opts.mode == GPT2L_MODE_TF32X3 ? kb_per_pair >= 16.0 : (d.N >= 8192 || (plain && kb_per_pair >= 96.0)))
-      dd.opts.cta_pair = 2;
-  }
+  dd.opts.cta_pair = choose_cta_pair(d, ctx->num_sms, ctx->max_pairs);
   GemmOp op;
   // Wide weight gradients (lm_head: N = 50304 against K = 768): the tensor core reads an MN-major A
   // operand about 20 % slower than a K-major one, and here A = in^T is tiny next to the GEMM. So
@@ -399,8 +382,10 @@ int gpt2_linear_forward_xent(float *logits, float *losses, float *lse, const flo
   if (d.opts.flags || d.opts.aux_op || d.opts.xent_lse || d.opts.force_simt || !logits || !in || !w || K <= 0 || N <= 0 ||
       !tma_eligible(d))
     return GPT2L_ERR_BAD_ARG;
-  // the statistics buffer's size follows the tiling, which follows the shape: plan first
+  // the statistics buffer's size and row stride follow the tiling, so the op that will be launched is planned first,
+  // with everything that decides its tiling settled
   GemmOp probe;
+  d.opts.cta_pair = choose_cta_pair(d, ctx->num_sms, ctx->max_pairs);
   d.xent_stats = reinterpret_cast<float *>(16);  // any non-null value: plan_op only looks at shapes
   d.xent_vocab = V;
   err = plan_op(d, ctx->num_sms, &probe);

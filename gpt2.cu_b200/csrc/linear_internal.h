@@ -294,6 +294,9 @@ bool tma_eligible(const GemmDesc &d);
 int build_op(const GemmDesc &d, int num_sms, GemmOp *op);
 // The host-only part of build_op (no tensor maps, no CUDA calls): shapes, tiling, descriptor bits.
 int plan_op(const GemmDesc &d, int num_sms, GemmOp *op);
+// opts.cta_pair with the choice that 0 leaves open settled: 1 (single CTAs) or 2 (CTA pairs). No CUDA calls. Whatever
+// needs the plan of a call before it is launched settles this first, because the tiling depends on it.
+int choose_cta_pair(const GemmDesc &d, int num_sms, int max_pairs);
 long long launch_count_value();
 // tile index inside an op -> (tile row, tile column, split); shared by the kernel and the host replay
 __host__ __device__ __forceinline__ void decode_local(int local, int tiles_m, int tiles_n, int band_m,

@@ -991,6 +991,25 @@ int plan_op(const GemmDesc &d, int num_sms, GemmOp *op) {
   return GPT2L_OK;
 }
 
+// 256 x 256 tiles of a CTA pair stage a third less operand data per flop. What that saves grows with the k-blocks a pair
+// works through; what it costs is a few microseconds of cluster launch and hand-shakes. TF32, 8192 rows (single CTAs / pairs,
+// us): 768 -> 3072 forward 75.9 / 71.6, 3072 -> 768 78.4 / 73.0 (125 k-blocks a pair), 768 -> 768 28.9 / 31.0 (31);
+// 768 -> 50304 1089 / 990. In 3xTF32 mode the operand split is a third less work per CTA as well: 328 / 248 and 350 / 254,
+// 125 / 96; 2048 rows 768 -> 2304 70 / 58 (23); 1024 x 1024 x 1024 37 / 35, its weight gradient 39.7 / 41.2 (7).
+int choose_cta_pair(const GemmDesc &d, int num_sms, int max_pairs) {
+  if (d.opts.cta_pair != 0) return d.opts.cta_pair;
+  if (d.opts.xent_lse || max_pairs <= 0 || max_pairs < num_sms / 2) return 1;
+  const long long rows = d.kind == GPT2L_OP_BACKWARD_WEIGHT ? d.K : d.M;
+  const long long cols = d.kind == GPT2L_OP_BACKWARD_INPUT ? d.K : d.N;
+  const long long red = d.kind == GPT2L_OP_FORWARD ? d.K : d.kind == GPT2L_OP_BACKWARD_INPUT ? d.N : d.M;
+  const double kb_per_pair = (double)((rows + 255) / 256) * ((cols + 255) / 256) * ((red + BK - 1) / BK) / max_pairs;
+  // (a TF32 pair drains its tile with four warps per CTA, not eight: an epilogue that does more than store, GELU or an
+  // operand, costs what the main loop gains; the MLP's six calls at 8192 rows: all on single CTAs 595 us, all on pairs
+  // 646, the three plain ones on pairs 577)
+  const bool plain = !d.opts.aux_op && !(d.opts.flags & GPT2L_EPI_GELU_DUAL);
+  return (d.opts.mode == GPT2L_MODE_TF32X3 ? kb_per_pair >= 16.0 : (d.N >= 8192 || (plain && kb_per_pair >= 96.0))) ? 2 : 1;
+}
+
 int build_op(const GemmDesc &d, int num_sms, GemmOp *op) {
   if (!d.out || !d.a || !d.b) return GPT2L_ERR_BAD_ARG;
   int e = plan_op(d, num_sms, op);

@@ -86,6 +86,44 @@ def test_fused_cross_entropy_against_float64(gpu, mode, shape):
     assert rel(dw, dw2) <= (1e-4 if mode == 1 else TOL[mode])
 
 
+# mode, M, K, N: shapes where CTA pairs and single CTAs take tiles of different widths, so that statistics sized or read by
+# any other plan than the launched one are those of other rows (or of an older call: the buffer is filled with such first)
+@pytest.mark.parametrize("mode,M,K,N", [(1, 128, 768, 16384), (1, 1056, 960, 2048), (1, 1544, 2048, 640), (1, 320, 1600, 3072),
+                                        (0, 256, 2048, 8192), (0, 32, 768, 8192), (0, 32, 768, 16384), (0, 64, 256, 50304),
+                                        (0, 700, 256, 8192), (0, 256, 1600, 8192), (0, 100, 128, 8192)])
+def test_statistics_are_read_as_they_were_written(gpu, mode, M, K, N):
+    gen = torch.Generator(device="cuda").manual_seed(M + K)
+
+    def loss_and_lse(x, w, tgt, V):
+        rows, (k, n) = x.shape[0], w.shape
+        logits = torch.empty((rows, n), device="cuda")
+        losses, lse = (torch.full((rows,), float("nan"), device="cuda") for _ in range(2))
+        gpu.check("forward_xent", gpu.forward_xent(logits, losses, lse, x, w, tgt, 1, rows, k, n, V, gpu.make_opts(mode=mode)))
+        torch.cuda.synchronize()
+        return losses, lse
+
+    def case(rows, k, n, scale):
+        x = torch.randn((rows, k), device="cuda", generator=gen) * scale
+        w = torch.randn((k, n), device="cuda", generator=gen) / k ** 0.5
+        return x, w, torch.randint(0, n - 13, (rows,), dtype=torch.int32, device="cuda", generator=gen)
+
+    big = case(2048, 768, 50304, 20.0)
+    loss_and_lse(*big, 50304 - 13)
+    del big
+    # neighbouring rows differ a lot: log-sum-exps of about log V + 0.1 and log V + 7
+    x, w, tgt = case(M, K, N, torch.tensor([0.5, 4.0], device="cuda").repeat(M // 2)[:, None])
+    V = N - 13
+    losses, lse = loss_and_lse(x, w, tgt, V)
+    z = (x.double() @ w.double())[:, :V]
+    lse64 = torch.logsumexp(z, dim=1)
+    # operands keep 10 mantissa bits (3xTF32: 21), sums are fp32: a logit is within c times the sum of its products'
+    # magnitudes, a log-sum-exp within the largest of its logits' errors and of its own fp32 sums (1e-4)
+    c = 2.0 ** -9 if mode == 0 else 2.0 ** -19
+    bound = (c + 2 * (K + 1) * 2.0 ** -24) * (x.abs().double() @ w.abs().double())[:, :V].amax(1) + 1e-4
+    assert bool(((lse.double() * np.log(2.0) - lse64).abs() <= bound).all())
+    assert bool(((losses.double() - (lse64 - z[torch.arange(M), tgt.long()])).abs() <= 2 * bound).all())
+
+
 def test_fused_cross_entropy_argument_checks(gpu):
     M, K, N, V = 128, 64, 256, 250
     x = torch.zeros((M, K), device="cuda")
@@ -139,3 +177,30 @@ def test_model_with_fused_cross_entropy_equals_the_separate_kernel(gpu, monkeypa
         for i in range(len(bounds) - 1):
             x, y = a[bounds[i]:bounds[i + 1]], b[bounds[i]:bounds[i + 1]]
             assert np.abs(x - y).max() <= 1e-5 * max(np.abs(y).max(), 1e-12), (kind, i, np.abs(x - y).max(), np.abs(y).max())
+
+
+def test_model_whose_lm_head_goes_to_cta_pairs(gpu, monkeypatch):
+    """3xTF32, 128 tokens, 16384 words: the lm_head's pairs take wider tiles than single CTAs would. Loss and gradients by the
+    statistics of the epilogue (the default) agree with the stand-alone kernel: both are fp32 sums over the same logits, so
+    they differ by roundings (a loss of 9.7 by a few of 1e-6) where statistics of other rows would differ by tenths."""
+    vocab, C, T = 16384, 768, 128
+    rng = np.random.default_rng(4)
+    tok, tgt = (torch.from_numpy(rng.integers(0, vocab, T).astype(np.int32)).cuda() for _ in range(2))
+    params, res = None, {}
+    for kind in ("separate", "stats"):
+        monkeypatch.setenv("GPT2_XENT", kind)
+        m = gpu.Model(vocab, vocab, 1, C // 64, C, T, 1, T, mode=1)
+        if params is None:
+            params = (rng.standard_normal(m.num_params) * 0.05).astype(np.float32)
+        m.set_params(params)
+        gpu.check("forward", m.forward(tok, tgt))
+        loss = m.mean_loss()
+        gpu.check("backward", m.backward())
+        torch.cuda.synchronize()
+        g = np.empty_like(params)
+        m.get_grads(g)
+        res[kind] = (loss, g)
+        m.close()
+    assert abs(res["stats"][0] - res["separate"][0]) <= 1e-5 * res["separate"][0]
+    a, b = res["stats"][1], res["separate"][1]
+    assert np.isfinite(a).all() and np.abs(a - b).max() <= 1e-4 * np.abs(b).max()
