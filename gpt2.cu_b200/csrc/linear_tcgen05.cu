@@ -831,6 +831,13 @@ static int encode_map_chunked(CUtensorMap *map, const float *base, uint64_t inne
 
 static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
+// Relative time of a plan by the bytes its busiest unit stages: waves of tiles of `per` k-blocks, plus 6 k-blocks of fixed
+// overhead a tile (pipeline fill, epilogue); splits pay an extra pass over the output (two k-blocks' worth since the partials
+// go out as reduce-adds of the copy engine).
+static double bytes_cost(double waves, int per, int splits, int tile_rows, int bn) {
+  return waves * (per + 6.0 + (splits > 1 ? 2.0 : 0.0)) * (double)(tile_rows + bn);
+}
+
 // Picks the tile width and the number of reduction splits. Single CTAs in TF32 mode: by the time they should take, in
 // ns, from what was measured inside the kernel at 256 rows and over the GEMM set at 8192:
 //   - a k-block costs the loader and issuer 270 whatever the width (a 128 x 256 tile's MMAs 280); with the whole chip at
@@ -854,8 +861,9 @@ static void choose_tiling(int Mc, int Nc, int kb_total, int num_sms, int forced_
   const int cand[3] = {256, 128, 64};
   for (int ci = 0; ci < 3; ++ci) {
     const int bn = cand[ci];
-    if (pair && bn < 128) continue;         // each CTA of a pair holds bn / 2 >= 64 columns of B
-    if (bn > 64 && bn / 2 >= Nc) continue;  // tile twice as wide as the matrix
+    const int narrowest = pair ? 128 : 64;  // each CTA of a pair holds bn / 2 >= 64 columns of B
+    if (bn < narrowest) continue;
+    if (bn > narrowest && bn / 2 >= Nc) continue;  // tile twice as wide as the matrix
     const int tiles = tiles_m * ceil_div(Nc, bn);
     const double drain = bn == 256 ? 5200.0 : (bn == 128 ? 3500.0 : 2700.0);
     const int smax = forced_splits > 0 ? forced_splits : (kb_total < 32 ? kb_total : 32);
@@ -873,9 +881,7 @@ static void choose_tiling(int Mc, int Nc, int kb_total, int num_sms, int forced_
         cost = (waves - 1.0) * (body > drain ? body : drain) + body + drain;
         if (s > 1) cost += fixed_order ? 4000.0 + out_bytes * s / 3000.0 : 1500.0 + out_bytes * s / 8000.0;
       } else {
-        // + 6 k-blocks of fixed per-tile overhead (pipeline fill, epilogue); splits pay an extra pass over the
-        // output (two k-blocks' worth since the partials go out as reduce-adds of the copy engine)
-        cost = waves * (per + 6.0 + (s > 1 ? 2.0 : 0.0)) * (double)(tile_rows + bn);
+        cost = bytes_cost(waves, per, s, tile_rows, bn);
       }
       if (cost < best - 1e-9) {
         best = cost;
@@ -996,18 +1002,38 @@ int plan_op(const GemmDesc &d, int num_sms, GemmOp *op) {
 // us): 768 -> 3072 forward 75.9 / 71.6, 3072 -> 768 78.4 / 73.0 (125 k-blocks a pair), 768 -> 768 28.9 / 31.0 (31);
 // 768 -> 50304 1089 / 990. In 3xTF32 mode the operand split is a third less work per CTA as well: 328 / 248 and 350 / 254,
 // 125 / 96; 2048 rows 768 -> 2304 70 / 58 (23); 1024 x 1024 x 1024 37 / 35, its weight gradient 39.7 / 41.2 (7).
+// Above those lines the two plans are compared, over 140 shapes of 36 - 16000 rows and 64 - 38000 columns:
+//   - in 3xTF32 mode both plans' tiles must be 256 wide (pairs with 128: 3380 x 2280 x 620 102 / 130, 1936 x 14408 x 100
+//     78 / 104; single CTAs with 128: six shapes, 67 / 62 to 137 / 163);
+//   - the bytes that the busiest CTA stages must be fewer by a tenth. Where both plans fill their tiles the ratio is 0.67; it
+//     nears one where half of the pair's 256 rows or a last wave is empty (128 x 3212 x 11824 3xTF32 105 / 154, ratio 1.3;
+//     12992 x 288 x 3704 TF32 weight gradient 74 / 82, 0.92);
+//   - and a tile four k-blocks long (5772 x 64 from 12668 rows: 140 / 151; 30500 x 2744 from 100: 213 / 193).
 int choose_cta_pair(const GemmDesc &d, int num_sms, int max_pairs) {
   if (d.opts.cta_pair != 0) return d.opts.cta_pair;
   if (d.opts.xent_lse || max_pairs <= 0 || max_pairs < num_sms / 2) return 1;
+  const bool x3 = d.opts.mode == GPT2L_MODE_TF32X3;
   const long long rows = d.kind == GPT2L_OP_BACKWARD_WEIGHT ? d.K : d.M;
   const long long cols = d.kind == GPT2L_OP_BACKWARD_INPUT ? d.K : d.N;
   const long long red = d.kind == GPT2L_OP_FORWARD ? d.K : d.kind == GPT2L_OP_BACKWARD_INPUT ? d.N : d.M;
-  const double kb_per_pair = (double)((rows + 255) / 256) * ((cols + 255) / 256) * ((red + BK - 1) / BK) / max_pairs;
+  if (cols <= 64) return 1;  // half of the narrowest pair tile would be empty
+  if (!x3 && d.N >= 8192) return 2;
   // (a TF32 pair drains its tile with four warps per CTA, not eight: an epilogue that does more than store, GELU or an
   // operand, costs what the main loop gains; the MLP's six calls at 8192 rows: all on single CTAs 595 us, all on pairs
   // 646, the three plain ones on pairs 577)
-  const bool plain = !d.opts.aux_op && !(d.opts.flags & GPT2L_EPI_GELU_DUAL);
-  return (d.opts.mode == GPT2L_MODE_TF32X3 ? kb_per_pair >= 16.0 : (d.N >= 8192 || (plain && kb_per_pair >= 96.0))) ? 2 : 1;
+  if (!x3 && (d.opts.aux_op || (d.opts.flags & GPT2L_EPI_GELU_DUAL))) return 1;
+  const double kb_per_pair = (double)((rows + 255) / 256) * ((cols + 255) / 256) * ((red + BK - 1) / BK) / max_pairs;
+  if (kb_per_pair < (x3 ? 16.0 : 96.0)) return 1;
+  GemmDesc t = d;
+  GemmOp one, two;
+  t.opts.cta_pair = 1;
+  if (plan_op(t, num_sms, &one) != GPT2L_OK) return 1;  // (the call itself reports the error)
+  t.opts.cta_pair = 2;
+  if (plan_op(t, num_sms, &two) != GPT2L_OK) return 1;
+  if ((x3 && (one.bn < MAX_BN || two.bn < MAX_BN)) || two.kb_per_split < 4) return 1;
+  const double bytes_one = bytes_cost(ceil_div(one.n_tiles, num_sms), one.kb_per_split, one.splits, BM, one.bn);
+  const double bytes_two = bytes_cost(ceil_div(two.n_tiles, max_pairs), two.kb_per_split, two.splits, 2 * BM, two.bn) / 2;
+  return bytes_two <= 0.9 * bytes_one ? 2 : 1;
 }
 
 int build_op(const GemmDesc &d, int num_sms, GemmOp *op) {

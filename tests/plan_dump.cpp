@@ -1,0 +1,24 @@
+// Prints the tiling that the library plans for calls read from standard input, on a machine with or without a GPU:
+//   mode kind M K N split_k cta_pair deterministic aux gelu stats  ->  error pair bn splits kb_per_split tiles_n
+#include <cstdio>
+
+#include "linear_internal.h"
+
+int main() {
+  constexpr int SMS = 148, PAIRS = 74;
+  int mode, kind, M, K, N, split, pair, det, aux, gelu, stats;
+  while (scanf("%d %d %d %d %d %d %d %d %d %d %d", &mode, &kind, &M, &K, &N, &split, &pair, &det, &aux, &gelu, &stats) == 11) {
+    float *any = reinterpret_cast<float *>(16);  // plans look at shapes and options, not at memory
+    g2l::GemmDesc d = {};
+    d.kind = kind; d.M = M; d.K = K; d.N = N;
+    d.out = any; d.a = any; d.b = any;
+    d.opts.mode = mode; d.opts.split_k = split; d.opts.cta_pair = pair; d.opts.deterministic = det;
+    if (aux) { d.opts.aux_op = aux; d.opts.aux = any; }
+    if (gelu) { d.opts.flags = GPT2L_EPI_GELU_DUAL; d.opts.out2 = any; }
+    if (stats) { d.xent_stats = any; d.xent_vocab = N; }
+    d.opts.cta_pair = g2l::choose_cta_pair(d, SMS, PAIRS);
+    g2l::GemmOp op;
+    const int e = g2l::plan_op(d, SMS, &op);
+    printf("%d %d %d %d %d %d\n", e, op.pair, op.bn, op.splits, op.kb_per_split, op.tiles_n);
+  }
+}

@@ -34,6 +34,28 @@ def test_every_direction_against_float64(gpu, mode, M, K, N):
     assert rel(db, D.sum(0)) <= 1e-5
 
 
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("pair", [0, 1, 2])
+@pytest.mark.parametrize("split,det", [(0, 0), (0, 1), (5, 0), (5, 1)])
+@pytest.mark.parametrize("M,K,N", [(1000, 132, 64), (516, 260, 36), (2048, 64, 4)])
+def test_narrow_outputs_against_float64(gpu, mode, pair, split, det, M, K, N):
+    """outputs narrower than a pair's narrowest tile, in one part or several, added by the copy engine or in fixed order"""
+    gen = torch.Generator(device="cuda").manual_seed(M + N)
+    x, w, dy = (torch.randn(s, device="cuda", generator=gen) for s in ((M, K), (K, N), (M, N)))
+    y, dx, dw, db = (torch.full(s, float("nan"), device="cuda") for s in ((M, N), (M, K), (K, N), (N,)))
+    o = gpu.make_opts(mode=mode, cta_pair=pair, split_k=split, deterministic=det)
+    gpu.check("forward", gpu.forward(y, x, w, None, 1, M, K, N, o))
+    gpu.check("backward_input", gpu.backward_input(dx, dy, w, 1, M, K, N, o))
+    gpu.check("backward_weight", gpu.backward_weight(dw, db, dy, x, 1, M, K, N, o))
+    torch.cuda.synchronize()
+    X, W, D = x.double(), w.double(), dy.double()
+    # operands keep 10 mantissa bits (3xTF32: 21), sums are fp32: within c times the sum of the products' magnitudes
+    c = 2.0 ** -9 if mode == 0 else 2.0 ** -19
+    for got, a, b, terms in ((y, X, W, K), (dx, D, W.t(), N), (dw, X.t(), D, M)):
+        assert bool(((got.double() - a @ b).abs() <= (c + 2 * (terms + 1) * 2.0 ** -24) * (a.abs() @ b.abs())).all())
+    assert bool(((db.double() - D.sum(0)).abs() <= 2 * M * 2.0 ** -24 * D.abs().sum(0)).all())
+
+
 class _View:
     def __init__(self, ptr, count):
         self.__cuda_array_interface__ = {"shape": (count,), "typestr": "<f4", "data": (ptr, False), "version": 3}

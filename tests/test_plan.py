@@ -1,0 +1,55 @@
+"""The automatic choices of a linear-layer call (CTA pairs, tile width, splits), planned for 148 SMs without a GPU."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+LIBDIR = os.path.join(ROOT, "gpt2.cu_b200", "lib")
+
+
+@pytest.fixture(scope="module")
+def plans(built, tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("plan") / "plan_dump")
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    r = subprocess.run([nvcc, "-std=c++17", "-I", os.path.join(ROOT, "include"), "-I", os.path.join(ROOT, "gpt2.cu_b200", "csrc"),
+                        os.path.join(ROOT, "tests", "plan_dump.cpp"), "-o", exe, "-L", LIBDIR, "-lgpt2_linear",
+                        f"-Xlinker=-rpath={LIBDIR}"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+    def run(calls):
+        """calls: dicts of mode, kind, M, K, N and options -> one dict per call"""
+        fields = ("mode", "kind", "M", "K", "N", "split", "pair", "det", "aux", "gelu", "stats")
+        text = "\n".join(" ".join(str(c.get(f, 0)) for f in fields) for c in calls)
+        out = subprocess.run([exe], input=text + "\n", capture_output=True, text=True, check=True).stdout
+        return [dict(zip(("err", "pair", "bn", "splits", "per", "tiles_n"), map(int, line.split()))) for line in out.splitlines()]
+
+    return run
+
+
+FORWARD, BACKWARD_INPUT, BACKWARD_WEIGHT = 0, 1, 2
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+def test_narrow_outputs_keep_their_reduction_split(plans, mode):
+    deep = dict(mode=mode, kind=BACKWARD_WEIGHT, M=16384, K=5120, N=64)
+    deeper = dict(deep, K=768)
+    asked = dict(deep, split=7)
+    for p, at_least in zip(plans([deep, deeper, asked]), (7, 24, 7)):
+        assert p["err"] == 0 and p["pair"] == 0 and p["bn"] == 64 and p["splits"] >= at_least
+    # a caller who asks for pairs gets their narrowest tile, split as asked or as the rows need it
+    (p, q) = plans([dict(asked, pair=2), dict(deeper, pair=2)])
+    assert p["pair"] == q["pair"] == 1 and p["bn"] == q["bn"] == 128
+    assert p["splits"] == 7 and q["splits"] > 8
+
+
+def test_pairs_where_they_stage_less(plans):
+    rows = 8192
+    calls = [dict(mode=1, kind=k, M=rows, K=a, N=b) for k in range(3) for a, b in ((768, 3072), (3072, 768), (768, 2304))]
+    calls += [dict(mode=0, kind=k, M=rows, K=768, N=n) for k in range(3) for n in (3072, 50304)]
+    assert all(p["pair"] == 1 and p["bn"] == 256 for p in plans(calls))
+    # 128 rows leave half of a pair's tile empty; 100 columns more than half of one; two k-blocks are all hand-shake
+    calls = [dict(mode=1, kind=BACKWARD_INPUT, M=128, K=3212, N=11824), dict(mode=1, kind=BACKWARD_INPUT, M=1936, K=100, N=14408),
+             dict(mode=1, kind=FORWARD, M=12668, K=64, N=5772)]
+    assert all(p["pair"] == 0 for p in plans(calls))
