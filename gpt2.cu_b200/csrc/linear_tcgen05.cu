@@ -1008,6 +1008,9 @@ int plan_op(const GemmDesc &d, int num_sms, GemmOp *op) {
 //   - the bytes that the busiest CTA stages must be fewer by a tenth. Where both plans fill their tiles the ratio is 0.67; it
 //     nears one where half of the pair's 256 rows or a last wave is empty (128 x 3212 x 11824 3xTF32 105 / 154, ratio 1.3;
 //     12992 x 288 x 3704 TF32 weight gradient 74 / 82, 0.92);
+//   - no 3xTF32 accumulator may sum a longer chain than the single CTAs', because that sum bounds the mode's error (forward
+//     3620 x 4724 x 860, 30 k-blocks against 148: 6.6e-6 / 3.3e-5 for 311 / 282 us; weight gradient 4320 x 1096 x 3200, 27
+//     against 135: 6.1e-6 / 3.0e-5 for 278 / 236);
 //   - and a tile four k-blocks long (5772 x 64 from 12668 rows: 140 / 151; 30500 x 2744 from 100: 213 / 193).
 int choose_cta_pair(const GemmDesc &d, int num_sms, int max_pairs) {
   if (d.opts.cta_pair != 0) return d.opts.cta_pair;
@@ -1031,6 +1034,7 @@ int choose_cta_pair(const GemmDesc &d, int num_sms, int max_pairs) {
   t.opts.cta_pair = 2;
   if (plan_op(t, num_sms, &two) != GPT2L_OK) return 1;
   if ((x3 && (one.bn < MAX_BN || two.bn < MAX_BN)) || two.kb_per_split < 4) return 1;
+  if (x3 && two.kb_per_split > one.kb_per_split) return 1;
   const double bytes_one = bytes_cost(ceil_div(one.n_tiles, num_sms), one.kb_per_split, one.splits, BM, one.bn);
   const double bytes_two = bytes_cost(ceil_div(two.n_tiles, max_pairs), two.kb_per_split, two.splits, 2 * BM, two.bn) / 2;
   return bytes_two <= 0.9 * bytes_one ? 2 : 1;

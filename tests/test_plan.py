@@ -1,5 +1,6 @@
 """The automatic choices of a linear-layer call (CTA pairs, tile width, splits), planned for 148 SMs without a GPU."""
 import os
+import random
 import shutil
 import subprocess
 
@@ -53,3 +54,13 @@ def test_pairs_where_they_stage_less(plans):
     calls = [dict(mode=1, kind=BACKWARD_INPUT, M=128, K=3212, N=11824), dict(mode=1, kind=BACKWARD_INPUT, M=1936, K=100, N=14408),
              dict(mode=1, kind=FORWARD, M=12668, K=64, N=5772)]
     assert all(p["pair"] == 0 for p in plans(calls))
+
+
+def test_pairs_sum_no_longer_chains_in_3xtf32(plans):
+    """the accumulation bounds this mode's error, so the choice that is left open never lengthens it"""
+    rng = random.Random(3)
+    calls = [dict(mode=1, kind=FORWARD, M=3620, K=4724, N=860), dict(mode=1, kind=BACKWARD_WEIGHT, M=4320, K=1096, N=3200)]
+    calls += [dict(mode=1, kind=rng.randrange(3), **{k: 4 * round(2 ** rng.uniform(4, 12)) for k in "MKN"}) for _ in range(3000)]
+    chosen, single = plans(calls), plans([dict(c, pair=1) for c in calls])
+    assert sum(p["pair"] for p in chosen) > 500
+    assert all(p["per"] <= q["per"] for p, q in zip(chosen, single))
