@@ -187,7 +187,10 @@ __device__ __forceinline__ bool xform_tile(const GemmScalars *op, const Tile &tc
       const int lin_lo = xmode == 2 ? (A_TILE_BYTES >> 4) : 0;
       const int lin_f4 = walk_b ? (A_TILE_BYTES >> 4) : stage_f4;
       constexpr int T = NUM_XFORM_WARPS * 32;
-      for (int i = lin_lo + x; i < lin_f4; i += 8 * T) split_hi_lo<8>(reinterpret_cast<float4 *>(stage), rg.lo, i, T, lin_f4);
+      // (the step kernel is out of registers: eight values in flight go through local memory there, 8 x 512 tokens of an MLP's
+      // six GEMMs 1404 us, one at a time 1081)
+      constexpr int V = MEGA ? 1 : 8;
+      for (int i = lin_lo + x; i < lin_f4; i += V * T) split_hi_lo<V>(reinterpret_cast<float4 *>(stage), rg.lo, i, T, lin_f4);
     }
     if (rewrites) fence_proxy_async_smem();
     __syncwarp();
