@@ -160,51 +160,68 @@ __device__ __forceinline__ bool row_ln_bwd(const GemmOp *op, int tile, int w8, i
   const int wtid = w8 * 32 + lane;
   const int r0 = tile * op->rows_per_tile;
   const int r1 = min(M, r0 + op->rows_per_tile);
+  // Columns of a row (times 128) that are in registers at once, beside the column sums. Up to six, the whole row; the three
+  // rows of a wider one would go through local memory (C = 1024: 110 - 320 us a tile of 64 rows, and two layers' step of
+  // 4 x 512 tokens 3425 - 3850 us, whatever way the compiler spilled), so it is fetched again for the second half of the
+  // work, from the L2 (3320 us).
+  constexpr int HELD = K4 <= 6 ? K4 : K4 / 2;
+  static_assert(K4 % HELD == 0, "whole parts");
   float4 dw[K4], db[K4];
 #pragma unroll
   for (int k = 0; k < K4; ++k) dw[k] = db[k] = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int row = r0 + w8; row < r1; row += NUM_WORKER_WARPS) {
-    float4 nh[K4], g[K4], o[K4];
+    float4 nh[HELD], g[HELD], o[HELD];
     const float *x = a.in1 + (long long)row * C;
     const float *go = a.in0 + (long long)row * C;
     float *gi = a.out0 + (long long)row * C;
     const float mu = a.in3[row], rs = a.in4[row];
     // all three rows in one round trip: the residual gradient this row is added to comes with its inputs
+    auto fetch = [&](int k0) {
 #pragma unroll
-    for (int k = 0; k < K4; ++k) {
-      const int c = 4 * (lane + 32 * k);
-      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-      nh[k] = c < C ? *reinterpret_cast<const float4 *>(x + c) : zero;   // x for now
-      g[k] = c < C ? *reinterpret_cast<const float4 *>(go + c) : zero;
-      o[k] = c < C ? *reinterpret_cast<const float4 *>(gi + c) : zero;
-    }
+      for (int k = 0; k < HELD; ++k) {
+        const int c = 4 * (lane + 32 * (k0 + k));
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 xv = c < C ? *reinterpret_cast<const float4 *>(x + c) : zero;
+        g[k] = c < C ? *reinterpret_cast<const float4 *>(go + c) : zero;
+        o[k] = c < C ? *reinterpret_cast<const float4 *>(gi + c) : zero;
+        nh[k] = make_float4((xv.x - mu) * rs, (xv.y - mu) * rs, (xv.z - mu) * rs, (xv.w - mu) * rs);
+      }
+    };
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
-    for (int k = 0; k < K4; ++k) {
-      const int c = 4 * (lane + 32 * k);
-      if (c < C) {
-        const float4 xv = nh[k];
-        nh[k] = make_float4((xv.x - mu) * rs, (xv.y - mu) * rs, (xv.z - mu) * rs, (xv.w - mu) * rs);
-        const float4 wv = *reinterpret_cast<const float4 *>(a.in2 + c);
-        const float4 dn = make_float4(g[k].x * wv.x, g[k].y * wv.y, g[k].z * wv.z, g[k].w * wv.w);
-        s1 += dn.x + dn.y + dn.z + dn.w;
-        s2 += dn.x * nh[k].x + dn.y * nh[k].y + dn.z * nh[k].z + dn.w * nh[k].w;
+    for (int k0 = 0; k0 < K4; k0 += HELD) {
+      fetch(k0);
+#pragma unroll
+      for (int k = 0; k < HELD; ++k) {
+        const int c = 4 * (lane + 32 * (k0 + k));
+        if (c < C) {
+          const float4 wv = *reinterpret_cast<const float4 *>(a.in2 + c);
+          const float4 dn = make_float4(g[k].x * wv.x, g[k].y * wv.y, g[k].z * wv.z, g[k].w * wv.w);
+          s1 += dn.x + dn.y + dn.z + dn.w;
+          s2 += dn.x * nh[k].x + dn.y * nh[k].y + dn.z * nh[k].z + dn.w * nh[k].w;
+        }
       }
     }
     s1 = rw_warp_sum(s1) / C;
     s2 = rw_warp_sum(s2) / C;
+    if (HELD < K4) asm volatile("" ::: "memory");  // fetched again, not kept
 #pragma unroll
-    for (int k = 0; k < K4; ++k) {
-      const int c = 4 * (lane + 32 * k);
-      if (c < C) {
-        const float4 wv = *reinterpret_cast<const float4 *>(a.in2 + c);
-        o[k].x += (g[k].x * wv.x - s1 - nh[k].x * s2) * rs;
-        o[k].y += (g[k].y * wv.y - s1 - nh[k].y * s2) * rs;
-        o[k].z += (g[k].z * wv.z - s1 - nh[k].z * s2) * rs;
-        o[k].w += (g[k].w * wv.w - s1 - nh[k].w * s2) * rs;
-        *reinterpret_cast<float4 *>(gi + c) = o[k];
-        dw[k].x += g[k].x * nh[k].x; dw[k].y += g[k].y * nh[k].y; dw[k].z += g[k].z * nh[k].z; dw[k].w += g[k].w * nh[k].w;
-        db[k].x += g[k].x; db[k].y += g[k].y; db[k].z += g[k].z; db[k].w += g[k].w;
+    for (int k0 = 0; k0 < K4; k0 += HELD) {
+      if (HELD < K4) fetch(k0);
+#pragma unroll
+      for (int k = 0; k < HELD; ++k) {
+        const int c = 4 * (lane + 32 * (k0 + k));
+        if (c < C) {
+          const float4 wv = *reinterpret_cast<const float4 *>(a.in2 + c);
+          o[k].x += (g[k].x * wv.x - s1 - nh[k].x * s2) * rs;
+          o[k].y += (g[k].y * wv.y - s1 - nh[k].y * s2) * rs;
+          o[k].z += (g[k].z * wv.z - s1 - nh[k].z * s2) * rs;
+          o[k].w += (g[k].w * wv.w - s1 - nh[k].w * s2) * rs;
+          *reinterpret_cast<float4 *>(gi + c) = o[k];
+          float4 &w = dw[k0 + k], &b = db[k0 + k];
+          w.x += g[k].x * nh[k].x; w.y += g[k].y * nh[k].y; w.z += g[k].z * nh[k].z; w.w += g[k].w * nh[k].w;
+          b.x += g[k].x; b.y += g[k].y; b.z += g[k].z; b.w += g[k].w;
+        }
       }
     }
   }

@@ -139,3 +139,36 @@ def test_step_with_unsatisfiable_dependency_ends_cleanly(gpu):
     assert abs(m.mean_loss() - z["losses"][0]) <= 1e-4
     st2.close()
     m.close()
+
+
+@pytest.mark.parametrize("n_embd", [832, 1024, 1280])
+def test_wide_rows_equal_the_separate_launches(gpu, monkeypatch, n_embd):
+    """Rows of more than 768 columns (6.5, 8 and 10 parts of 128), whose layernorm backward fetches its inputs twice: one
+    layer, 3xTF32, without the update. Loss and gradients agree up to the order of the sums (bounds as at 768 above)."""
+    monkeypatch.setenv("GPT2_ATTENTION", "flash")
+    vocab, B, T = 512, 2, 128
+    params = gpt2_ref.to_flat(gpt2_ref.init_params(vocab, T, 1, n_embd // 64, n_embd), 1, vocab)
+    rng = np.random.default_rng(6)
+    tok, tgt = (torch.from_numpy(rng.integers(0, vocab, B * T).astype(np.int32)).cuda() for _ in range(2))
+    res = []
+    for step in (False, True):
+        m = gpu.Model(vocab, vocab, 1, n_embd // 64, n_embd, T, B, T, mode=1)
+        m.set_params(params)
+        if step:
+            st = gpu.Step(m, tok, tgt, with_update=False)
+            assert st.run() == 0
+            torch.cuda.synchronize()
+            assert st.status() == 0
+            st.close()
+        else:
+            assert m.forward(tok, tgt) == 0 and m.backward() == 0
+        g = np.empty_like(params)
+        loss = m.mean_loss()
+        m.get_grads(g)
+        bounds = m.offsets() + [m.num_params]
+        res.append((loss, g))
+        m.close()
+    assert abs(res[0][0] - res[1][0]) <= 5e-6
+    for lo, hi in zip(bounds, bounds[1:]):
+        a, b = res[1][1][lo:hi], res[0][1][lo:hi]
+        assert np.isfinite(a).all() and np.abs(a - b).max() <= 5e-4 * max(np.abs(b).max(), 1e-12), (lo, np.abs(a - b).max())
