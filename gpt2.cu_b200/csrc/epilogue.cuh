@@ -47,7 +47,7 @@ __device__ __forceinline__ bool colsum_global_tile(const GemmScalars *op, const 
     unsigned seen = 0u;
     int okl = 1;
     if (lane == 0) okl = wait_deps(op, m_tile, ctrl, p, seen) ? 1 : 0;
-    if (__shfl_sync(0xffffffffu, okl, 0) == 0) return false;
+    if (!from_lane0(okl)) return false;
   }
   const int bn = op->bn;
   const int g_groups = bn >> 2;          // float4 column groups of the tile: 16, 32 or 64
@@ -95,7 +95,7 @@ __device__ __forceinline__ bool epilogue_tile(const GemmScalars *op, const GemmO
   if (lane == 0)
     okl = PAIR ? wait_bar_cluster(smem_u32(&ctrl->tmem_full[as]), aph, ctrl, p, SITE_TMEM_FULL, op->op_index, as, G2L_TMEM_FULL_BACKOFF)
                : wait_bar(smem_u32(&ctrl->tmem_full[as]), aph, ctrl, p, SITE_TMEM_FULL, op->op_index, as, G2L_TMEM_FULL_BACKOFF);
-  if (__shfl_sync(0xffffffffu, okl, 0) == 0) return false;
+  if (!from_lane0(okl)) return false;
   tc_fence_after();
 
   const int bn = op->bn;

@@ -111,7 +111,7 @@ __device__ __forceinline__ bool xform_tile(const GemmScalars *op, const Tile &tc
     const bool cs_kb = do_colsum && (!spread || (kb % op->tiles_m) == tc.m_tile);
     // (these warps rewrite or sum every stage here, so each is on the ring's critical path: no back-off)
     if (lane == 0) okl = wait_bar(smem_u32(&ctrl->full[s]), ph, ctrl, p, SITE_SMEM_FULL, op->op_index, s);
-    ok = __shfl_sync(0xffffffffu, okl, 0) != 0;
+    ok = from_lane0(okl);
     if (!ok) break;
     uint8_t *stage = ring_ptr + s * rg.stride;
     if (xmode == 2 && kb == tc.kb0) {
@@ -339,7 +339,7 @@ __device__ __noinline__ bool row_op_tile(const GemmOp *op, const Tile &tc, int w
   const int rb = op->op_kind == OPK_ADAMW ? 0 : (int)(((long long)tile * rpt) >> 7);
   int okl = 1;
   if (lane == 0) okl = wait_deps(op, rb, ctrl, p, deps_done) ? 1 : 0;
-  if (__shfl_sync(0xffffffffu, okl, 0) == 0) return false;
+  if (!from_lane0(okl)) return false;
   const int wtid = w8 * 32 + lane;
   bool ok = true;
   switch (op->op_kind) {
@@ -403,7 +403,7 @@ __device__ __forceinline__ bool cta_sync(Ctrl *ctrl, const LaunchParams &p, Attn
     okl = wait_bar(bar, ap.cta_phase & 1u, ctrl, p, SITE_CTA_SYNC, op, (int)ap.cta_phase, 20) ? 1 : 0;
   }
   ++ap.cta_phase;
-  return __shfl_sync(0xffffffffu, okl, 0) != 0;
+  return from_lane0(okl);
 }
 
 // One attention tile (128 rows of one head of one sequence) run by the whole CTA between two GEMM tiles:
@@ -425,7 +425,7 @@ __device__ __noinline__ bool attention_tile_mode(const GemmOp *op, int grb, int 
       ap.deps_done = 0u;
     }
     if (lane == 0) okl = wait_deps(op, grb, ctrl, p, ap.deps_done) ? 1 : 0;
-    if (__shfl_sync(0xffffffffu, okl, 0) == 0) return false;
+    if (!from_lane0(okl)) return false;
     fence_proxy_async_all();  // the operands were written with plain stores; TMA reads them next
   }
   if (!cta_sync(ctrl, p, ap, op->op_index, lane)) return false;
@@ -588,7 +588,7 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
         }
         int okl = 1;
         if (lane == 0) okl = wait_deps(op, tc.m_tile, ctrl, p, deps_done) ? 1 : 0;
-        ok = __shfl_sync(0xffffffffu, okl, 0) != 0;
+        ok = from_lane0(okl);
         if (!ok) break;
         fence_proxy_async_all();  // producers wrote with plain stores; TMA reads next
       }

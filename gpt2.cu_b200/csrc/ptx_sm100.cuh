@@ -174,6 +174,12 @@ __device__ __forceinline__ bool elect_one() {
       : "=r"(p));
   return p != 0;
 }
+// Lane 0's verdict on a wait, for its whole warp (converged). The __syncwarp orders what the other lanes, and a thread elected
+// among them, do next behind what lane 0 acquired: a shuffle orders no memory.
+__device__ __forceinline__ bool from_lane0(int verdict) {
+  __syncwarp();
+  return __shfl_sync(0xffffffffu, verdict, 0) != 0;
+}
 // D[tmem] (+)= A[smem] . B[smem], TF32 inputs, fp32 accumulate. One thread issues.
 __device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                          uint32_t idesc, uint32_t accumulate) {

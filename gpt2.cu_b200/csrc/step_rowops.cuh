@@ -28,7 +28,7 @@ struct RowSync {
       okl = wait_bar(bar, phase & 1u, ctrl, p, SITE_ROW_SYNC, op, (int)phase, 20) ? 1 : 0;
     }
     ++phase;
-    return __shfl_sync(0xffffffffu, okl, 0) != 0;
+    return from_lane0(okl);
   }
 };
 
