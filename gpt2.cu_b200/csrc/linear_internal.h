@@ -350,6 +350,12 @@ cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
 int attention_flash_build_maps(FlashMaps *maps, const float *qkv, const float *dout, int B, int T, int C, int NH);
 
 // --- linear_simt.cu ---
+struct SimtPlan {
+  int bm, bn;      // tile: 128 x 128, 128 x 64 or 64 x 64
+  int parts;       // reduction parts = CTAs of a cluster
+  int k_per_part;  // a multiple of 16
+};
+SimtPlan simt_plan(int Mc, int Nc, int Kc, int sms, int max_parts);  // no CUDA calls
 int launch_simt(const GemmDesc &d, cudaStream_t stream);
 int launch_colsum(float *out, const float *x, int rows, int cols, cudaStream_t stream);
 // zeroes a[0 .. n) (16-byte aligned, n a multiple of four; may be empty) and b[0 .. nb)

@@ -6,6 +6,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "linear_internal.h"
 #include "ptx_sm100.cuh"
 
@@ -31,7 +33,7 @@ namespace g2l {
 constexpr int SK = 16;  // k per slab
 constexpr int SIMT_STAGES = 3;
 constexpr int SIMT_THREADS = 256;
-constexpr int SIMT_MAX_PARTS = 16;  // (clusters of more than 8 need the kernel's consent)
+constexpr int SIMT_MAX_PARTS = 16;  // (clusters of more than 8 need the kernel's consent and a device that can place them)
 
 template <int BMT, int BNT>
 struct SimtCfg {
@@ -285,26 +287,18 @@ int launch_transpose(float *dst, const float *src, int rows, int cols, cudaStrea
   return e == cudaSuccess ? GPT2L_OK : GPT2L_ERR_CUDA;
 }
 
-namespace {
-
-struct SimtPlan {
-  int bm, bn;      // tile: 128 x 128, 128 x 64 or 64 x 64
-  int parts;       // reduction parts = CTAs of a cluster
-  int k_per_part;  // a multiple of SK
-};
-
 // The tile and the split whose busiest SM has the least to do. Smaller tiles cost more per product (shared-memory
 // reads per FMA), a CTA that has its SM to itself reaches 73 % of what two reach together (23.7 against 50 TFLOP/s x
 // 96 / 148 SMs), and a part pays for filling its ring and for the exchange of the partial tiles, counted as
-// SIMT_FIXED_K more k.
-SimtPlan simt_plan(int Mc, int Nc, int Kc, int sms) {
+// SIMT_FIXED_K more k. `max_parts`: the largest cluster the device can place.
+SimtPlan simt_plan(int Mc, int Nc, int Kc, int sms, int max_parts) {
   constexpr double SIMT_FIXED_K = 48.0;
   static const struct { int bm, bn; double per_product; } tile[3] = {{128, 128, 1.0}, {128, 64, 1.2}, {64, 64, 1.6}};
   SimtPlan best = {128, 128, 1, 0};
   double best_cost = 1e300;
   for (const auto &t : tile) {
     const double tiles = (double)((Mc + t.bm - 1) / t.bm) * ((Nc + t.bn - 1) / t.bn);
-    for (int parts = 1; parts <= SIMT_MAX_PARTS; parts *= 2) {
+    for (int parts = 1; parts <= max_parts; parts *= 2) {
       const int per = ((Kc + parts - 1) / parts + SK - 1) / SK * SK;
       if (parts > 1 && (long long)per * (parts - 1) >= Kc) break;  // an empty part
       const double ctas_per_sm = ceil(tiles * parts / sms);
@@ -319,12 +313,53 @@ SimtPlan simt_plan(int Mc, int Nc, int Kc, int sms) {
   return best;
 }
 
-int current_sms() {
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-    return 148;
-  return sms;
+namespace {
+
+using SimtKernel = void (*)(float *, const float *, const float *, const float *, int, int, int, long long, long long, long long,
+                            long long, long long, int, int);
+
+cudaLaunchConfig_t simt_config(cudaLaunchAttribute *attr, long long tiles, int parts, size_t smem, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)tiles, 1, (unsigned)parts);
+  cfg.blockDim = dim3(SIMT_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = (unsigned)parts;
+  cfg.attrs = attr;
+  cfg.numAttrs = parts > 1 ? 1 : 0;
+  return cfg;
+}
+
+int simt_attributes(SimtKernel kernel, int smem) {
+  // (per device and cheap: set every time rather than tracking which devices have seen it)
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+                 cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess
+             ? GPT2L_OK
+             : GPT2L_ERR_CUDA;
+}
+
+// The largest cluster of the 128 x 128 kernel, the one with the most shared memory, that the current device can place (a
+// partition of a GPU may not hold 16 CTAs side by side); asked once per device.
+int simt_max_parts(int dev) {
+  constexpr int DEVICES = 16;
+  static std::atomic<int> known[DEVICES];
+  const bool keep = dev >= 0 && dev < DEVICES;
+  if (keep && known[dev].load(std::memory_order_relaxed) > 0) return known[dev].load(std::memory_order_relaxed);
+  constexpr int smem = SimtCfg<128, 128>::SMEM;
+  SimtKernel kernel = gpt2_linear_simt_kernel<128, 128, true, true>;
+  int parts = simt_attributes(kernel, smem) == GPT2L_OK ? SIMT_MAX_PARTS : 1;
+  for (; parts > 1; parts /= 2) {
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = simt_config(attr, 1, parts, smem, nullptr);
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0) break;
+    (void)cudaGetLastError();
+  }
+  if (keep) known[dev].store(parts, std::memory_order_relaxed);
+  return parts;
 }
 
 template <int BMT, int BNT>
@@ -333,24 +368,11 @@ int simt_launch(const SimtPlan &pl, float *c, const float *a, const float *b, co
   using G = SimtCfg<BMT, BNT>;
   const long long tiles_n = (Nc + BNT - 1) / BNT, tiles = tiles_n * ((Mc + BMT - 1) / BMT);
   if (tiles > 0x7fffffffll) return GPT2L_ERR_TOO_LARGE;
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  cfg.gridDim = dim3((unsigned)tiles, 1, (unsigned)pl.parts);
-  cfg.blockDim = dim3(SIMT_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = G::SMEM;
-  cfg.stream = stream;
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = (unsigned)pl.parts;
-  cfg.attrs = attr;
-  cfg.numAttrs = pl.parts > 1 ? 1 : 0;
-  auto kernel = ak == 1 ? (bj == 1 ? gpt2_linear_simt_kernel<BMT, BNT, true, false> : gpt2_linear_simt_kernel<BMT, BNT, true, true>)
+  const SimtKernel kernel = ak == 1 ? (bj == 1 ? gpt2_linear_simt_kernel<BMT, BNT, true, false> : gpt2_linear_simt_kernel<BMT, BNT, true, true>)
                         : gpt2_linear_simt_kernel<BMT, BNT, false, false>;
-  // (per device and cheap: set every time rather than tracking which devices have seen it)
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM) != cudaSuccess ||
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-    return GPT2L_ERR_CUDA;
+  if (simt_attributes(kernel, G::SMEM)) return GPT2L_ERR_CUDA;
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = simt_config(attr, tiles, pl.parts, G::SMEM, stream);
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, c, a, b, bias, Mc, Nc, Kc, ai, ak, bk, bj, (long long)Nc,
                                            pl.k_per_part, (int)tiles_n);
   count_launch();
@@ -377,7 +399,11 @@ int launch_simt(const GemmDesc &d, cudaStream_t stream) {
     default:
       return GPT2L_ERR_BAD_ARG;
   }
-  SimtPlan pl = simt_plan(Mc, Nc, Kc, current_sms());
+  int dev = -1, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+    sms = 148;
+  const SimtPlan pl = simt_plan(Mc, Nc, Kc, sms, simt_max_parts(dev));
   int e;
   if (pl.bn == 128) e = simt_launch<128, 128>(pl, d.out, d.a, d.b, bias, Mc, Nc, Kc, ai, ak, bk, bj, stream);
   else if (pl.bm == 128) e = simt_launch<128, 64>(pl, d.out, d.a, d.b, bias, Mc, Nc, Kc, ai, ak, bk, bj, stream);

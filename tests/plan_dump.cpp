@@ -1,10 +1,23 @@
 // Prints the tiling that the library plans for calls read from standard input, on a machine with or without a GPU:
 //   mode kind M K N split_k cta_pair deterministic aux gelu stats  ->  error pair bn splits kb_per_split tiles_n
+// With the argument "simt", the CUDA-core GEMM's plan instead:
+//   Mc Nc Kc max_parts  ->  tile rows, tile columns, parts, k per part
 #include <cstdio>
+#include <cstring>
 
 #include "linear_internal.h"
 
-int main() {
+static int simt() {
+  int Mc, Nc, Kc, max_parts;
+  while (scanf("%d %d %d %d", &Mc, &Nc, &Kc, &max_parts) == 4) {
+    const g2l::SimtPlan p = g2l::simt_plan(Mc, Nc, Kc, 148, max_parts);
+    printf("%d %d %d %d\n", p.bm, p.bn, p.parts, p.k_per_part);
+  }
+  return 0;
+}
+
+int main(int argc, char **argv) {
+  if (argc > 1 && !strcmp(argv[1], "simt")) return simt();
   constexpr int SMS = 148, PAIRS = 74;
   int mode, kind, M, K, N, split, pair, det, aux, gelu, stats;
   while (scanf("%d %d %d %d %d %d %d %d %d %d %d", &mode, &kind, &M, &K, &N, &split, &pair, &det, &aux, &gelu, &stats) == 11) {

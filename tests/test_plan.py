@@ -11,20 +11,29 @@ LIBDIR = os.path.join(ROOT, "gpt2.cu_b200", "lib")
 
 
 @pytest.fixture(scope="module")
-def plans(built, tmp_path_factory):
+def plan_dump(built, tmp_path_factory):
     exe = str(tmp_path_factory.mktemp("plan") / "plan_dump")
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     r = subprocess.run([nvcc, "-std=c++17", "-I", os.path.join(ROOT, "include"), "-I", os.path.join(ROOT, "gpt2.cu_b200", "csrc"),
                         os.path.join(ROOT, "tests", "plan_dump.cpp"), "-o", exe, "-L", LIBDIR, "-lgpt2_linear",
                         f"-Xlinker=-rpath={LIBDIR}"], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr[-2000:]
+    return exe
 
+
+def _lines(command, rows):
+    text = "\n".join(" ".join(map(str, r)) for r in rows) + "\n"
+    out = subprocess.run(command, input=text, capture_output=True, text=True, check=True).stdout
+    return [tuple(map(int, line.split())) for line in out.splitlines()]
+
+
+@pytest.fixture(scope="module")
+def plans(plan_dump):
     def run(calls):
         """calls: dicts of mode, kind, M, K, N and options -> one dict per call"""
         fields = ("mode", "kind", "M", "K", "N", "split", "pair", "det", "aux", "gelu", "stats")
-        text = "\n".join(" ".join(str(c.get(f, 0)) for f in fields) for c in calls)
-        out = subprocess.run([exe], input=text + "\n", capture_output=True, text=True, check=True).stdout
-        return [dict(zip(("err", "pair", "bn", "splits", "per", "tiles_n"), map(int, line.split()))) for line in out.splitlines()]
+        rows = _lines([plan_dump], [[c.get(f, 0) for f in fields] for c in calls])
+        return [dict(zip(("err", "pair", "bn", "splits", "per", "tiles_n"), r)) for r in rows]
 
     return run
 
@@ -64,3 +73,15 @@ def test_pairs_sum_no_longer_chains_in_3xtf32(plans):
     chosen, single = plans(calls), plans([dict(c, pair=1) for c in calls])
     assert sum(p["pair"] for p in chosen) > 500
     assert all(p["per"] <= q["per"] for p, q in zip(chosen, single))
+
+
+@pytest.mark.parametrize("max_parts", [1, 2, 4, 8, 16])
+def test_cuda_core_splits_fit_the_device(plan_dump, max_parts):
+    """no more parts than the largest cluster the device can place, none of them empty, nothing left out"""
+    rng = random.Random(5)
+    shapes = [(768, 256, 50257), (1, 1, 1)] + [tuple(round(2 ** rng.uniform(0, 15)) for _ in range(3)) for _ in range(500)]
+    plans = _lines([plan_dump, "simt"], [s + (max_parts,) for s in shapes])
+    for (_, _, depth), (bm, bn, parts, per) in zip(shapes, plans):
+        assert 1 <= parts <= max_parts and per % 16 == 0 and (bm, bn) in ((128, 128), (128, 64), (64, 64))
+        assert per * (parts - 1) < depth <= per * parts
+    assert plans[0][2] == max_parts  # 12 or 24 tiles, 50257 deep: as many parts as there may be
