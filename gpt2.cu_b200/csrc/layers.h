@@ -5,6 +5,18 @@
 
 namespace g2l {
 
+// Blocks of the fp32 attention kernels, one per head, sequence and 64-row tile, in one dimension (the only one of a grid that
+// is not limited to 65535): heads fastest, then sequences, so that the tiles of one length run together.
+constexpr int ATT_TILE = 64;
+struct AttBlock {
+  int head, seq, tile;
+};
+inline long long att_blocks(int B, int T, int NH) { return (long long)B * NH * (((long long)T + ATT_TILE - 1) / ATT_TILE); }
+__host__ __device__ inline AttBlock att_block(unsigned index, int B, int NH) {
+  const unsigned per_head = index / NH;
+  return {(int)(index % NH), (int)(per_head % B), (int)(per_head / B)};
+}
+
 int embedding_forward(float *out, const int *tokens, const float *wte, const float *wpe, int B, int T, int C, int Vp,
                       cudaStream_t s);
 // zeroes g[0 .. head) and `pairs` ranges of two_c floats, the k-th at first + (k / 2) * layer + (k % 2) * second, the last at

@@ -2,9 +2,12 @@
 //   mode kind M K N split_k cta_pair deterministic aux gelu stats  ->  error pair bn splits kb_per_split tiles_n
 // With the argument "simt", the CUDA-core GEMM's plan instead:
 //   Mc Nc Kc max_parts  ->  tile rows, tile columns, parts, k per part
+// With "attention", the grid of the fp32 attention kernels and its blocks (of large ones the first and the last):
+//   B T NH  ->  number of blocks, then head, sequence and tile of each
 #include <cstdio>
 #include <cstring>
 
+#include "layers.h"
 #include "linear_internal.h"
 
 static int simt() {
@@ -16,7 +19,22 @@ static int simt() {
   return 0;
 }
 
+static int attention() {
+  int B, T, NH;
+  while (scanf("%d %d %d", &B, &T, &NH) == 3) {
+    const long long n = g2l::att_blocks(B, T, NH);
+    printf("%lld", n);
+    for (long long i = 0; i < n; i += n > 4096 ? n - 1 : 1) {
+      const g2l::AttBlock k = g2l::att_block((unsigned)i, B, NH);
+      printf(" %d %d %d", k.head, k.seq, k.tile);
+    }
+    printf("\n");
+  }
+  return 0;
+}
+
 int main(int argc, char **argv) {
+  if (argc > 1 && !strcmp(argv[1], "attention")) return attention();
   if (argc > 1 && !strcmp(argv[1], "simt")) return simt();
   constexpr int SMS = 148, PAIRS = 74;
   int mode, kind, M, K, N, split, pair, det, aux, gelu, stats;

@@ -85,3 +85,15 @@ def test_cuda_core_splits_fit_the_device(plan_dump, max_parts):
         assert 1 <= parts <= max_parts and per % 16 == 0 and (bm, bn) in ((128, 128), (128, 64), (64, 64))
         assert per * (parts - 1) < depth <= per * parts
     assert plans[0][2] == max_parts  # 12 or 24 tiles, 50257 deep: as many parts as there may be
+
+
+def test_fp32_attention_covers_every_sequence_length(plan_dump):
+    """one block per head, sequence and 64 rows, in the grid dimension that holds more than 65535"""
+    (row,) = _lines([plan_dump, "attention"], [(3, 129, 2)])
+    blocks = [row[i:i + 3] for i in range(1, len(row), 3)]
+    assert row[0] == len(blocks) == 18
+    assert blocks == [(h, b, t) for t in range(3) for b in range(3) for h in range(2)]
+    for B, T, NH in ((1, 65535 * 64 + 1, 1), (2, 1 << 23, 3)):
+        (row,) = _lines([plan_dump, "attention"], [(B, T, NH)])
+        tiles = -(-T // 64)
+        assert row[0] == B * NH * tiles < 2 ** 31 and row[1:] == (0, 0, 0, NH - 1, B - 1, tiles - 1)
