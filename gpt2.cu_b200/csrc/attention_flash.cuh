@@ -115,7 +115,7 @@ __device__ __forceinline__ bool w_wait(uint32_t bar, uint32_t parity, FlashCtrl 
                                        int lane) {
   int okl = 1;
   if (lane == 0) okl = f_wait(bar, parity, ctrl, a, site) ? 1 : 0;
-  return from_lane0(okl);
+  return __shfl_sync(0xffffffffu, okl, 0) != 0;
 }
 
 __device__ __forceinline__ float ex2(float x) {

@@ -95,7 +95,7 @@ __device__ __forceinline__ bool epilogue_tile(const GemmScalars *op, const GemmO
   if (lane == 0)
     okl = PAIR ? wait_bar_cluster(smem_u32(&ctrl->tmem_full[as]), aph, ctrl, p, SITE_TMEM_FULL, op->op_index, as, G2L_TMEM_FULL_BACKOFF)
                : wait_bar(smem_u32(&ctrl->tmem_full[as]), aph, ctrl, p, SITE_TMEM_FULL, op->op_index, as, G2L_TMEM_FULL_BACKOFF);
-  if (!from_lane0(okl)) return false;
+  if (__shfl_sync(0xffffffffu, okl, 0) == 0) return false;
   tc_fence_after();
 
   const int bn = op->bn;

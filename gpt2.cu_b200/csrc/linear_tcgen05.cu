@@ -111,7 +111,7 @@ __device__ __forceinline__ bool xform_tile(const GemmScalars *op, const Tile &tc
     const bool cs_kb = do_colsum && (!spread || (kb % op->tiles_m) == tc.m_tile);
     // (these warps rewrite or sum every stage here, so each is on the ring's critical path: no back-off)
     if (lane == 0) okl = wait_bar(smem_u32(&ctrl->full[s]), ph, ctrl, p, SITE_SMEM_FULL, op->op_index, s);
-    ok = from_lane0(okl);
+    ok = __shfl_sync(0xffffffffu, okl, 0) != 0;
     if (!ok) break;
     uint8_t *stage = ring_ptr + s * rg.stride;
     if (xmode == 2 && kb == tc.kb0) {

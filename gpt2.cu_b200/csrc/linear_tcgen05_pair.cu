@@ -306,7 +306,7 @@ gpt2_linear_tcgen05_pair_kernel(const __grid_constant__ GemmOp op0, const Launch
           int okl = 1;
           if (lane == 0)
             okl = wait_bar(smem_u32(&ctrl->full[s]), ph, ctrl, p, SITE_SMEM_FULL, op->op_index, s, X3 ? 0 : 64);
-          ok = from_lane0(okl);
+          ok = __shfl_sync(0xffffffffu, okl, 0) != 0;
           if (!ok) break;
           uint8_t *stage = ring_ptr + s * STAGE_STRIDE;
           const bool walk_b = do_colsum && kb % op->tiles_dec == tc.m_tile;

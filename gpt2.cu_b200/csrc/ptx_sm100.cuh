@@ -174,8 +174,10 @@ __device__ __forceinline__ bool elect_one() {
       : "=r"(p));
   return p != 0;
 }
-// Lane 0's verdict on a wait, for its whole warp (converged). The __syncwarp orders what the other lanes, and a thread elected
-// among them, do next behind what lane 0 acquired: a shuffle orders no memory.
+// Lane 0's verdict on a wait for other warps or CTAs, for its whole warp (converged). The __syncwarp orders what the other
+// lanes, and a thread elected among them, do next behind what lane 0 acquired: a shuffle orders no memory. (The waits of
+// every k-block and attention step keep the bare shuffle: they hand over stages and accumulators that the copy engine or the
+// tensor core has completed before the barrier's phase ends, and the __syncwarp cost 1 - 2 % of an attention pass.)
 __device__ __forceinline__ bool from_lane0(int verdict) {
   __syncwarp();
   return __shfl_sync(0xffffffffu, verdict, 0) != 0;
