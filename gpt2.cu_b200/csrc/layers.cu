@@ -526,10 +526,11 @@ __device__ __forceinline__ float4 att_quad(const unsigned long long (&a)[2], flo
 }
 
 __global__ void __launch_bounds__(ATT_THREADS, 2)
-attention_forward_kernel(float *out, float *lse, const float *qkv, int B, int T, int C, int NH) {
+attention_forward_kernel(float *out, float *lse, const float *qkv, int T, int C, int NH) {
   extern __shared__ __align__(16) float sm[];
   float *sq = sm, *sk = sm + ATILE, *sv = sm + 2 * ATILE, *sp = sm + 3 * ATILE;
-  const AttBlock blk = att_block(blockIdx.x, B, NH);
+  const AttBlock blk = att_block(blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x, NH);
+  if (blk.tile > (T - 1) / AT) return;
   const int h = blk.head, b = blk.seq, q0 = ((T - 1) / AT - blk.tile) * AT;  // the longest rows first
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
   const float scale = 0.125f;  // 1 / sqrt(64)
@@ -591,10 +592,11 @@ attention_forward_kernel(float *out, float *lse, const float *qkv, int B, int T,
 // dS_ij = p_ij (dO_i.V_j - delta_i), dQ_i = sum_j dS_ij K_j / 8
 __global__ void __launch_bounds__(ATT_THREADS, 2)
 attention_backward_dq_kernel(float *dqkv, const float *dout, const float *qkv, const float *lse, const float *delta,
-                             int B, int T, int C, int NH) {
+                             int T, int C, int NH) {
   extern __shared__ __align__(16) float sm[];
   float *sq = sm, *sg = sm + ATILE, *sk = sm + 2 * ATILE, *sv = sm + 3 * ATILE, *ss = sm + 4 * ATILE;
-  const AttBlock blk = att_block(blockIdx.x, B, NH);
+  const AttBlock blk = att_block(blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x, NH);
+  if (blk.tile > (T - 1) / AT) return;
   const int h = blk.head, b = blk.seq, q0 = ((T - 1) / AT - blk.tile) * AT;
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
   const float scale = 0.125f;
@@ -637,10 +639,11 @@ attention_backward_dq_kernel(float *dqkv, const float *dout, const float *qkv, c
 // dV_j = sum_i p_ij dO_i;  dK_j = sum_i dS_ij Q_i / 8: rows of a tile are keys, its columns the queries at or after them
 __global__ void __launch_bounds__(ATT_THREADS, 2)
 attention_backward_dkv_kernel(float *dqkv, const float *dout, const float *qkv, const float *lse, const float *delta,
-                              int B, int T, int C, int NH) {
+                              int T, int C, int NH) {
   extern __shared__ __align__(16) float sm[];
   float *sk = sm, *sv = sm + ATILE, *sq = sm + 2 * ATILE, *sg = sm + 3 * ATILE, *sp = sm + 4 * ATILE, *ss = sm + 5 * ATILE;
-  const AttBlock blk = att_block(blockIdx.x, B, NH);
+  const AttBlock blk = att_block(blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x, NH);
+  if (blk.tile > (T - 1) / AT) return;
   const int h = blk.head, b = blk.seq, k0 = blk.tile * AT;  // the keys most queries see first
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
   const float scale = 0.125f;
@@ -866,25 +869,22 @@ int attention_forward(float *out, float *lse, const float *qkv, int B, int T, in
   // (per device and cheap: set every time rather than tracking which devices have seen it)
   if (cudaFuncSetAttribute(attention_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return GPT2L_ERR_CUDA;
-  const long long blocks = att_blocks(B, T, NH);
-  if (blocks > 0x7fffffffll) return GPT2L_ERR_TOO_LARGE;
-  attention_forward_kernel<<<(unsigned)blocks, ATT_THREADS, smem, s>>>(out, lse, qkv, B, T, C, NH);
+  attention_forward_kernel<<<att_grid(B, T, NH), ATT_THREADS, smem, s>>>(out, lse, qkv, T, C, NH);
   return LAUNCH_OK();
 }
 int attention_backward(float *dqkv, float *delta, const float *dout, const float *out, const float *qkv,
                        const float *lse, int B, int T, int C, int NH, cudaStream_t s) {
   if (C != NH * HS) return GPT2L_ERR_BAD_ARG;
-  if (att_blocks(B, T, NH) > 0x7fffffffll) return GPT2L_ERR_TOO_LARGE;
   constexpr int smem_q = 5 * ATILE * (int)sizeof(float), smem_kv = 6 * ATILE * (int)sizeof(float);
   if (cudaFuncSetAttribute(attention_backward_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_q) != cudaSuccess ||
       cudaFuncSetAttribute(attention_backward_dkv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_kv) != cudaSuccess)
     return GPT2L_ERR_CUDA;
   const int e = attention_row_dot(delta, dout, out, B, T, C, NH, s);
   if (e) return e;
-  const unsigned blocks = (unsigned)att_blocks(B, T, NH);
-  attention_backward_dq_kernel<<<blocks, ATT_THREADS, smem_q, s>>>(dqkv, dout, qkv, lse, delta, B, T, C, NH);
+  const dim3 grid = att_grid(B, T, NH);
+  attention_backward_dq_kernel<<<grid, ATT_THREADS, smem_q, s>>>(dqkv, dout, qkv, lse, delta, T, C, NH);
   count_launch();
-  attention_backward_dkv_kernel<<<blocks, ATT_THREADS, smem_kv, s>>>(dqkv, dout, qkv, lse, delta, B, T, C, NH);
+  attention_backward_dkv_kernel<<<grid, ATT_THREADS, smem_kv, s>>>(dqkv, dout, qkv, lse, delta, T, C, NH);
   return LAUNCH_OK();
 }
 int adamw_update(float *p, float *m, float *v, const float *g, long long n, float lr, float b1, float b2, float eps,

@@ -5,16 +5,20 @@
 
 namespace g2l {
 
-// Blocks of the fp32 attention kernels, one per head, sequence and 64-row tile, in one dimension (the only one of a grid that
-// is not limited to 65535): heads fastest, then sequences, so that the tiles of one length run together.
+// Blocks of the fp32 attention kernels, one per head, sequence and 64-row tile in the three dimensions of a grid, so that the
+// tiles of one length run together. The third dimension holds 65535; the tiles of longer sequences (4 194 240 tokens) are
+// folded into the first (not always: a block's two divisions cost 0.3 us a kernel, 3 % of a short call).
 constexpr int ATT_TILE = 64;
 struct AttBlock {
-  int head, seq, tile;
+  int head, seq, tile;  // tile may lie past the last one where tiles are folded
 };
-inline long long att_blocks(int B, int T, int NH) { return (long long)B * NH * (((long long)T + ATT_TILE - 1) / ATT_TILE); }
-__host__ __device__ inline AttBlock att_block(unsigned index, int B, int NH) {
-  const unsigned per_head = index / NH;
-  return {(int)(index % NH), (int)(per_head % B), (int)(per_head / B)};
+inline dim3 att_grid(int B, int T, int NH) {
+  const unsigned tiles = ((unsigned)T + ATT_TILE - 1) / ATT_TILE, folds = (tiles + 65534u) / 65535u;
+  return dim3(NH * folds, B, (tiles + folds - 1) / folds);
+}
+__host__ __device__ inline AttBlock att_block(unsigned x, unsigned y, unsigned z, unsigned grid_x, unsigned NH) {
+  if (grid_x == NH) return {(int)x, (int)y, (int)z};
+  return {(int)(x % NH), (int)y, (int)(z * (grid_x / NH) + x / NH)};
 }
 
 int embedding_forward(float *out, const int *tokens, const float *wte, const float *wpe, int B, int T, int C, int Vp,

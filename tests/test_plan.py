@@ -88,12 +88,14 @@ def test_cuda_core_splits_fit_the_device(plan_dump, max_parts):
 
 
 def test_fp32_attention_covers_every_sequence_length(plan_dump):
-    """one block per head, sequence and 64 rows, in the grid dimension that holds more than 65535"""
+    """one block per head, sequence and 64 rows, heads fastest and tiles slowest; no more than 65535 in a grid's second and
+    third dimension"""
     (row,) = _lines([plan_dump, "attention"], [(3, 129, 2)])
-    blocks = [row[i:i + 3] for i in range(1, len(row), 3)]
-    assert row[0] == len(blocks) == 18
-    assert blocks == [(h, b, t) for t in range(3) for b in range(3) for h in range(2)]
-    for B, T, NH in ((1, 65535 * 64 + 1, 1), (2, 1 << 23, 3)):
+    blocks = [row[i:i + 3] for i in range(3, len(row), 3)]
+    assert row[:3] == (2, 3, 3) and blocks == [(h, b, t) for t in range(3) for b in range(3) for h in range(2)]
+    for B, T, NH, folds in ((1, 65535 * 64, 2, 1), (1, 65535 * 64 + 1, 1, 2), (2, 1 << 23, 3, 3)):
         (row,) = _lines([plan_dump, "attention"], [(B, T, NH)])
-        tiles = -(-T // 64)
-        assert row[0] == B * NH * tiles < 2 ** 31 and row[1:] == (0, 0, 0, NH - 1, B - 1, tiles - 1)
+        tiles, depth = -(-T // 64), row[2]
+        assert row[:2] == (NH * folds, B) and depth <= 65535 and tiles <= folds * depth < tiles + folds
+        layers = [[(h, b, t) for b in range(B) for t in range(folds * z, folds * z + folds) for h in range(NH)] for z in (0, depth - 1)]
+        assert [row[i:i + 3] for i in range(3, len(row), 3)] == layers[0] + layers[1]
