@@ -385,9 +385,9 @@ int gpt2_linear_forward_xent(float *logits, float *losses, float *lse, const flo
   // the statistics buffer's size and row stride follow the tiling, so the op that will be launched is planned first,
   // with everything that decides its tiling settled
   GemmOp probe;
-  d.opts.cta_pair = choose_cta_pair(d, ctx->num_sms, ctx->max_pairs);
   d.xent_stats = reinterpret_cast<float *>(16);  // any non-null value: plan_op only looks at shapes
   d.xent_vocab = V;
+  d.opts.cta_pair = choose_cta_pair(d, ctx->num_sms, ctx->max_pairs);
   err = plan_op(d, ctx->num_sms, &probe);
   if (err) return err;
   {

@@ -278,8 +278,6 @@ __device__ __forceinline__ float tf32_round(float x) {
   return __uint_as_float(r);
 }
 
-
-
 // 3xTF32: x = hi + lo with hi = x rounded to TF32, for N values of shared memory `step` float4 apart: all loads before the
 // first store, because a thread that waits out the latency of every value in turn (the compiler may not move a load past
 // a store it cannot tell apart) took 220 cycles per value.

@@ -759,50 +759,46 @@ zero_accumulated_kernel(float *g, long long head, float *first, long long second
 // launchers
 // ------------------------------------------------------------------------------------
 #define LAUNCH_OK() (count_launch(), cudaGetLastError() == cudaSuccess ? GPT2L_OK : GPT2L_ERR_CUDA)
-#define PDL_OK() (count_launch(), le == cudaSuccess ? GPT2L_OK : GPT2L_ERR_CUDA)
+// (for launch_pdl, which returns the launch's own error)
+static int launched(cudaError_t e) {
+  count_launch();
+  return e == cudaSuccess ? GPT2L_OK : GPT2L_ERR_CUDA;
+}
 
 int embedding_forward(float *out, const int *tokens, const float *wte, const float *wpe, int B, int T, int C, int Vp,
                       cudaStream_t s) {
-  cudaError_t le;
   const long long n = (long long)B * T * C;
-  le = launch_pdl(embedding_forward_kernel, cdiv(n, 256), 256, 0, s, out, tokens, wte, wpe, B * T, T, C, Vp);
-  return PDL_OK();
+  return launched(launch_pdl(embedding_forward_kernel, cdiv(n, 256), 256, 0, s, out, tokens, wte, wpe, B * T, T, C, Vp));
 }
 int zero_accumulated(float *g, long long head, float *first, long long second, long long layer, long long last, int pairs,
                      int two_c, cudaStream_t s) {
-  cudaError_t le;
-  le = launch_pdl(zero_accumulated_kernel, cdiv(head + (long long)pairs * two_c, 256), 256, 0, s, g, head, first, second, layer, last, pairs,
-                                                                                 two_c);
-  return PDL_OK();
+  return launched(launch_pdl(zero_accumulated_kernel, cdiv(head + (long long)pairs * two_c, 256), 256, 0, s, g, head, first,
+                             second, layer, last, pairs, two_c));
 }
 int embedding_backward(float *g_wte, float *g_wpe, const float *g, const int *tokens, int B, int T, int C, int Vp,
                        cudaStream_t s) {
-  cudaError_t le;
   const long long n = (long long)B * T * C;
-  le = launch_pdl(embedding_backward_kernel, cdiv(n, 256), 256, 0, s, g_wte, g_wpe, g, tokens, B * T, T, C, Vp);
-  return PDL_OK();
+  return launched(launch_pdl(embedding_backward_kernel, cdiv(n, 256), 256, 0, s, g_wte, g_wpe, g, tokens, B * T, T, C, Vp));
 }
 int layernorm_forward(float *out, float *mean, float *rstd, const float *in, const float *w, const float *b, int M,
                       int C, cudaStream_t s) {
-  cudaError_t le;
-#define LN_FWD(K4) le = launch_pdl(layernorm_forward_vec_kernel<K4>, cdiv(M, 8), 256, 0, s, out, mean, rstd, in, w, b, M, C)
-  if (C & 3) le = launch_pdl(layernorm_forward_kernel, cdiv(M, 8), 256, 0, s, out, mean, rstd, in, w, b, M, C);
-  else if (C <= 128) LN_FWD(1);
-  else if (C <= 256) LN_FWD(2);
-  else if (C <= 512) LN_FWD(4);
-  else if (C <= 768) LN_FWD(6);
-  else if (C <= 1024) LN_FWD(8);
-  else if (C <= 1280) LN_FWD(10);
-  else if (C <= 2048) LN_FWD(16);
-  else le = launch_pdl(layernorm_forward_kernel, cdiv(M, 8), 256, 0, s, out, mean, rstd, in, w, b, M, C);
-#undef LN_FWD
-  return PDL_OK();
+  auto launch = [&](auto kernel) {
+    return launched(launch_pdl(kernel, cdiv(M, 8), 256, 0, s, out, mean, rstd, in, w, b, M, C));
+  };
+  if ((C & 3) || C > 2048) return launch(layernorm_forward_kernel);
+  if (C <= 128) return launch(layernorm_forward_vec_kernel<1>);
+  if (C <= 256) return launch(layernorm_forward_vec_kernel<2>);
+  if (C <= 512) return launch(layernorm_forward_vec_kernel<4>);
+  if (C <= 768) return launch(layernorm_forward_vec_kernel<6>);
+  if (C <= 1024) return launch(layernorm_forward_vec_kernel<8>);
+  if (C <= 1280) return launch(layernorm_forward_vec_kernel<10>);
+  return launch(layernorm_forward_vec_kernel<16>);
 }
 int layernorm_backward(float *g_in, float *g_w, float *g_b, const float *g_out, const float *in, const float *w,
                        const float *mean, const float *rstd, int M, int C, cudaStream_t s) {
-  cudaError_t le;
-  // one block per resident slot (two per SM) where there are rows enough: every block then ends at about
-  // the same time, and the column sums meet in global memory only ~300 times; a row per warp where there are not
+  // At most one block per resident slot (two per SM), so that all end at about the same time and the column sums meet in global
+  // memory only ~300 times, and whole rounds of a row per warp: from 8 rows a slot on the rows of a block are rounded up to
+  // 16, 24, ..., which leaves up to half of the slots idle just past each line (2376 rows: 149 blocks of 16).
   static const int slots = [] {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -814,17 +810,17 @@ int layernorm_backward(float *g_in, float *g_w, float *g_b, const float *g_out, 
   const int blocks = cdiv(M, rows_per_block);
   const size_t smem = 4 * (size_t)C * sizeof(float);
   if (C & 3) return GPT2L_ERR_BAD_ARG;
-#define LN_BWD(K4) le = launch_pdl(layernorm_backward_kernel<K4>, blocks, 256, smem, s, g_in, g_w, g_b, g_out, in, w, mean, rstd, M, C, rows_per_block)
-  if (C <= 128) LN_BWD(1);
-  else if (C <= 256) LN_BWD(2);
-  else if (C <= 512) LN_BWD(4);
-  else if (C <= 768) LN_BWD(6);
-  else if (C <= 1024) LN_BWD(8);
-  else if (C <= 1280) LN_BWD(10);
-  else if (C <= 2048) LN_BWD(16);
-  else return GPT2L_ERR_TOO_LARGE;
-#undef LN_BWD
-  return PDL_OK();
+  auto launch = [&](auto kernel) {
+    return launched(launch_pdl(kernel, blocks, 256, smem, s, g_in, g_w, g_b, g_out, in, w, mean, rstd, M, C, rows_per_block));
+  };
+  if (C <= 128) return launch(layernorm_backward_kernel<1>);
+  if (C <= 256) return launch(layernorm_backward_kernel<2>);
+  if (C <= 512) return launch(layernorm_backward_kernel<4>);
+  if (C <= 768) return launch(layernorm_backward_kernel<6>);
+  if (C <= 1024) return launch(layernorm_backward_kernel<8>);
+  if (C <= 1280) return launch(layernorm_backward_kernel<10>);
+  if (C <= 2048) return launch(layernorm_backward_kernel<16>);
+  return GPT2L_ERR_TOO_LARGE;
 }
 int add_forward(float *out, const float *a, const float *b, long long n, cudaStream_t s) {
   add_kernel<<<cdiv((n + 3) / 4, 256), 256, 0, s>>>(out, a, b, n);
@@ -852,16 +848,12 @@ int softmax_xent(float *logits, float *losses, const int *targets, int M, int V,
 }
 int launch_xent_combine(float *lse, float *losses, const float *stats, int stride, const float *logits, long long ld,
                         const int *targets, int M, cudaStream_t s) {
-  cudaError_t le;
-  le = launch_pdl(xent_combine_kernel, cdiv(M, 8), 256, 0, s, lse, losses, reinterpret_cast<const float2 *>(stats), stride, logits, ld,
-                                                  targets, M);
-  return PDL_OK();
+  return launched(launch_pdl(xent_combine_kernel, cdiv(M, 8), 256, 0, s, lse, losses, reinterpret_cast<const float2 *>(stats),
+                             stride, logits, ld, targets, M));
 }
 int xent_grad_inplace(float *logits, const float *lse, const int *targets, int M, int V, int Vp, cudaStream_t s) {
-  cudaError_t le;
   if (Vp & 3) return GPT2L_ERR_BAD_ARG;
-  le = launch_pdl(xent_grad_inplace_kernel, M, 512, 0, s, logits, lse, targets, V, Vp, 1.f / (float)M);
-  return PDL_OK();
+  return launched(launch_pdl(xent_grad_inplace_kernel, M, 512, 0, s, logits, lse, targets, V, Vp, 1.f / (float)M));
 }
 int attention_forward(float *out, float *lse, const float *qkv, int B, int T, int C, int NH, cudaStream_t s) {
   if (C != NH * HS) return GPT2L_ERR_BAD_ARG;
@@ -889,15 +881,14 @@ int attention_backward(float *dqkv, float *delta, const float *dout, const float
 }
 int adamw_update(float *p, float *m, float *v, const float *g, long long n, float lr, float b1, float b2, float eps,
                  float wd, int t, cudaStream_t s) {
-  cudaError_t le;
   const float bc1 = 1.f - powf(b1, (float)t), bc2 = 1.f - powf(b2, (float)t);
   // all four buffers are offset alike from 256-byte aligned allocations, so p decides the alignment
   long long head = (long long)((16 - (reinterpret_cast<uintptr_t>(p) & 15)) & 15) / 4;
   if (head > n) head = n;
   const long long n4 = (n - head) / 4;
   const long long extra = n - 4 * n4;  // head + tail, at most 6
-  le = launch_pdl(adamw_kernel, cdiv(n4 + extra, 256), 256, 0, s, p, m, v, g, n, head, n4, lr, b1, b2, eps, wd, bc1, bc2);
-  return PDL_OK();
+  return launched(launch_pdl(adamw_kernel, cdiv(n4 + extra, 256), 256, 0, s, p, m, v, g, n, head, n4, lr, b1, b2, eps, wd, bc1,
+                             bc2));
 }
 
 }  // namespace g2l

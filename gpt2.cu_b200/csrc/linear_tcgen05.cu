@@ -10,8 +10,10 @@
 //               (128 x bn x 8 per instruction, 4 per k-block), commits to `empty[s]`, and
 //               after the last k-block commits to `tmem_full[acc]`.
 //   warps 2-5   operand transform: in 3xTF32 mode split each landed stage into hi + lo
-//               copies; in backward_weight they also add up the columns of the B block
-//               (the bias gradient) for the tile row that owns it.
+//               copies. In backward_weight they also add up columns of B (the bias gradient):
+//               every tile row takes the k-blocks with kb % tiles_m == its index, from the
+//               landed stages in 3xTF32 mode, from global memory beside the ring in TF32 mode.
+//               In launches that leave them without such work they join the epilogue.
 //   warps 6-9   epilogue: tcgen05.ld the accumulator (warp w reads TMEM lanes 32*(w%4)..),
 //               add bias / GELU dual store / split-K combine, store fp32, then publish the
 //               tile on the dependency counters with a release reduction.
@@ -53,8 +55,8 @@ using namespace ptx;
 // ------------------------------------------------------------------------------------
 // Shape of the operand ring. The step kernel runs ops of any width through one ring, whose stages are as large as the
 // widest tile's; a launch of one op packs its stages, so that narrow tiles get more of them: 8 for bn = 64, 6 for 128,
-// 4 for 256 (3xTF32, hi and lo copies: 4, 3, 2). A copy takes about a microsecond to land, and with four stages of
-// 24 KiB a k-block of a 128 x 64 tile took 0.44 us, a third more than its MMAs.
+// 4 for 256 (3xTF32, hi and lo copies: 4, 3, 2). A copy takes about a microsecond to land, ten times as long as a
+// 128 x 64 tile's MMAs of a k-block (196 cycles), so a narrow tile needs more of them under way.
 template <bool X3, bool MEGA>
 struct Ring {
   int stages;

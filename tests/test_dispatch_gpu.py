@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 
 # mode, M, K, N: 3xTF32 just under and over the line for pairs (16 k-blocks a pair) with ragged edges; TF32 over the line
-# for plain calls (96); short batches, whose forward is unsplit and whose input gradient is split
+# for plain calls (96); short batches, with and without a split of the reduction
 @pytest.mark.parametrize("mode,M,K,N", [(1, 1030, 768, 1028), (1, 2052, 1028, 1540), (0, 4100, 3072, 772), (0, 4096, 772, 3072),
                                         (0, 256, 768, 2304), (0, 200, 2304, 772), (0, 60, 64, 68)])
 def test_every_direction_against_float64(gpu, mode, M, K, N):
