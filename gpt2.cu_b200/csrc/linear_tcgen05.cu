@@ -590,7 +590,8 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
         }
         int okl = 1;
         if (lane == 0) okl = wait_deps(op, tc.m_tile, ctrl, p, deps_done) ? 1 : 0;
-        ok = from_lane0(okl);
+        // (only lists have dependencies; the __syncwarp cost the 3xTF32 kernel of one op 1.8 % of an attention pass)
+        ok = MEGA ? from_lane0(okl) : __shfl_sync(0xffffffffu, okl, 0) != 0;
         if (!ok) break;
         fence_proxy_async_all();  // producers wrote with plain stores; TMA reads next
       }
@@ -850,8 +851,10 @@ static double bytes_cost(double waves, int per, int splits, int tile_rows, int b
 //   - draining a tile takes 2700 / 3500 / 5200; it hides behind the next tile's k-blocks, if any;
 //   - a split adds the zeroing of the output (a launch of its own) and its reduce-adds; the fixed-order combine passes
 //     through the workspace and costs several times as much. (fc forward at 256 rows, whose GELU store rules out
-//     reduce-adds: six splits of 256 columns 18.0 us, none of 64 columns 14.6; qkv forward 12.0 + 1.7 for the zeroing with
-//     eight splits, 8.6 with none.)
+//     reduce-adds: six splits of 256 columns 18.0 us, none of 64 columns 14.6; qkv forward with its zeroing: eight splits 10.7,
+//     four, which this picks, 9.5, none 10.5.)
+// The same times hold inside a schedule: six GEMMs of an MLP of 8 x 64 tokens, C 768, by bytes 95.7 us, by time 87.9; with
+// fixed-order sums 237 and 109.
 // CTA pairs and 3xTF32, whose k-blocks cost several times more: the pair that needs the fewest (waves x per-tile work),
 // where a tile's cost follows the bytes it pulls per k-block.
 static void choose_tiling(int Mc, int Nc, int kb_total, int num_sms, int forced_splits, bool pair, bool by_time,
