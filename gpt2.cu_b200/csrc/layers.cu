@@ -525,13 +525,12 @@ __device__ __forceinline__ float4 att_quad(const unsigned long long (&a)[2], flo
                      __uint_as_float((uint32_t)a[1]) * scale, __uint_as_float((uint32_t)(a[1] >> 32)) * scale);
 }
 
+template <bool LONG>  // one of several launches (att_launch_tiles)
 __global__ void __launch_bounds__(ATT_THREADS, 2)
-attention_forward_kernel(float *out, float *lse, const float *qkv, int T, int C, int NH) {
+attention_forward_kernel(float *out, float *lse, const float *qkv, int T, int C, int NH, int last) {
   extern __shared__ __align__(16) float sm[];
   float *sq = sm, *sk = sm + ATILE, *sv = sm + 2 * ATILE, *sp = sm + 3 * ATILE;
-  const AttBlock blk = att_block(blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x, NH);
-  if (blk.tile > (T - 1) / AT) return;
-  const int h = blk.head, b = blk.seq, q0 = ((T - 1) / AT - blk.tile) * AT;  // the longest rows first
+  const int h = blockIdx.x, b = blockIdx.y, q0 = ((LONG ? last + 1 : gridDim.z) - 1 - blockIdx.z) * AT;  // the longest rows first
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
   const float scale = 0.125f;  // 1 / sqrt(64)
   const long long ld = 3LL * C;
@@ -590,14 +589,13 @@ attention_forward_kernel(float *out, float *lse, const float *qkv, int T, int C,
 }
 
 // dS_ij = p_ij (dO_i.V_j - delta_i), dQ_i = sum_j dS_ij K_j / 8
+template <bool LONG>  // one of several launches (att_launch_tiles)
 __global__ void __launch_bounds__(ATT_THREADS, 2)
 attention_backward_dq_kernel(float *dqkv, const float *dout, const float *qkv, const float *lse, const float *delta,
-                             int T, int C, int NH) {
+                             int T, int C, int NH, int last) {
   extern __shared__ __align__(16) float sm[];
   float *sq = sm, *sg = sm + ATILE, *sk = sm + 2 * ATILE, *sv = sm + 3 * ATILE, *ss = sm + 4 * ATILE;
-  const AttBlock blk = att_block(blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x, NH);
-  if (blk.tile > (T - 1) / AT) return;
-  const int h = blk.head, b = blk.seq, q0 = ((T - 1) / AT - blk.tile) * AT;
+  const int h = blockIdx.x, b = blockIdx.y, q0 = ((LONG ? last + 1 : gridDim.z) - 1 - blockIdx.z) * AT;
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
   const float scale = 0.125f;
   const long long ld = 3LL * C, vbase = ((long long)b * NH + h) * T;
@@ -637,14 +635,13 @@ attention_backward_dq_kernel(float *dqkv, const float *dout, const float *qkv, c
 }
 
 // dV_j = sum_i p_ij dO_i;  dK_j = sum_i dS_ij Q_i / 8: rows of a tile are keys, its columns the queries at or after them
+template <bool LONG>  // one of several launches (att_launch_tiles)
 __global__ void __launch_bounds__(ATT_THREADS, 2)
 attention_backward_dkv_kernel(float *dqkv, const float *dout, const float *qkv, const float *lse, const float *delta,
-                              int T, int C, int NH) {
+                              int T, int C, int NH, int first) {
   extern __shared__ __align__(16) float sm[];
   float *sk = sm, *sv = sm + ATILE, *sq = sm + 2 * ATILE, *sg = sm + 3 * ATILE, *sp = sm + 4 * ATILE, *ss = sm + 5 * ATILE;
-  const AttBlock blk = att_block(blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x, NH);
-  if (blk.tile > (T - 1) / AT) return;
-  const int h = blk.head, b = blk.seq, k0 = blk.tile * AT;  // the keys most queries see first
+  const int h = blockIdx.x, b = blockIdx.y, k0 = (blockIdx.z + (LONG ? first : 0)) * AT;  // the keys most queries see first
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
   const float scale = 0.125f;
   const long long ld = 3LL * C, vbase = ((long long)b * NH + h) * T;
@@ -855,29 +852,52 @@ int xent_grad_inplace(float *logits, const float *lse, const int *targets, int M
   if (Vp & 3) return GPT2L_ERR_BAD_ARG;
   return launched(launch_pdl(xent_grad_inplace_kernel, M, 512, 0, s, logits, lse, targets, V, Vp, 1.f / (float)M));
 }
-int attention_forward(float *out, float *lse, const float *qkv, int B, int T, int C, int NH, cudaStream_t s) {
-  if (C != NH * HS) return GPT2L_ERR_BAD_ARG;
+template <bool LONG>
+static int attention_forward_launches(float *out, float *lse, const float *qkv, int B, int T, int C, int NH, cudaStream_t s) {
   constexpr int smem = 4 * ATILE * (int)sizeof(float);
   // (per device and cheap: set every time rather than tracking which devices have seen it)
-  if (cudaFuncSetAttribute(attention_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+  if (cudaFuncSetAttribute(attention_forward_kernel<LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return GPT2L_ERR_CUDA;
-  attention_forward_kernel<<<att_grid(B, T, NH), ATT_THREADS, smem, s>>>(out, lse, qkv, T, C, NH);
-  return LAUNCH_OK();
+  int err = GPT2L_OK;
+  for (int first = 0, n; err == GPT2L_OK && (n = att_launch_tiles(T, first)) > 0; first += n) {
+    attention_forward_kernel<LONG><<<dim3(NH, B, n), ATT_THREADS, smem, s>>>(out, lse, qkv, T, C, NH, (T - 1) / AT - first);
+    err = LAUNCH_OK();
+  }
+  return err;
+}
+template <bool LONG>
+static int attention_backward_launches(float *dqkv, const float *delta, const float *dout, const float *qkv, const float *lse,
+                                       int B, int T, int C, int NH, cudaStream_t s) {
+  constexpr int smem_q = 5 * ATILE * (int)sizeof(float), smem_kv = 6 * ATILE * (int)sizeof(float);
+  auto dq = attention_backward_dq_kernel<LONG>;
+  auto dkv = attention_backward_dkv_kernel<LONG>;
+  if (cudaFuncSetAttribute(dq, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_q) != cudaSuccess ||
+      cudaFuncSetAttribute(dkv, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_kv) != cudaSuccess)
+    return GPT2L_ERR_CUDA;
+  int err = GPT2L_OK;
+  for (int first = 0, n; err == GPT2L_OK && (n = att_launch_tiles(T, first)) > 0; first += n) {
+    const dim3 grid(NH, B, n);
+    dq<<<grid, ATT_THREADS, smem_q, s>>>(dqkv, dout, qkv, lse, delta, T, C, NH, (T - 1) / AT - first);
+    count_launch();
+    dkv<<<grid, ATT_THREADS, smem_kv, s>>>(dqkv, dout, qkv, lse, delta, T, C, NH, first);
+    err = LAUNCH_OK();
+  }
+  return err;
+}
+static bool att_long(int T) { return att_launch_tiles(T, 65535) > 0; }
+
+int attention_forward(float *out, float *lse, const float *qkv, int B, int T, int C, int NH, cudaStream_t s) {
+  if (C != NH * HS) return GPT2L_ERR_BAD_ARG;
+  return att_long(T) ? attention_forward_launches<true>(out, lse, qkv, B, T, C, NH, s)
+                     : attention_forward_launches<false>(out, lse, qkv, B, T, C, NH, s);
 }
 int attention_backward(float *dqkv, float *delta, const float *dout, const float *out, const float *qkv,
                        const float *lse, int B, int T, int C, int NH, cudaStream_t s) {
   if (C != NH * HS) return GPT2L_ERR_BAD_ARG;
-  constexpr int smem_q = 5 * ATILE * (int)sizeof(float), smem_kv = 6 * ATILE * (int)sizeof(float);
-  if (cudaFuncSetAttribute(attention_backward_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_q) != cudaSuccess ||
-      cudaFuncSetAttribute(attention_backward_dkv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_kv) != cudaSuccess)
-    return GPT2L_ERR_CUDA;
   const int e = attention_row_dot(delta, dout, out, B, T, C, NH, s);
   if (e) return e;
-  const dim3 grid = att_grid(B, T, NH);
-  attention_backward_dq_kernel<<<grid, ATT_THREADS, smem_q, s>>>(dqkv, dout, qkv, lse, delta, T, C, NH);
-  count_launch();
-  attention_backward_dkv_kernel<<<grid, ATT_THREADS, smem_kv, s>>>(dqkv, dout, qkv, lse, delta, T, C, NH);
-  return LAUNCH_OK();
+  return att_long(T) ? attention_backward_launches<true>(dqkv, delta, dout, qkv, lse, B, T, C, NH, s)
+                     : attention_backward_launches<false>(dqkv, delta, dout, qkv, lse, B, T, C, NH, s);
 }
 int adamw_update(float *p, float *m, float *v, const float *g, long long n, float lr, float b1, float b2, float eps,
                  float wd, int t, cudaStream_t s) {

@@ -5,20 +5,14 @@
 
 namespace g2l {
 
-// Blocks of the fp32 attention kernels, one per head, sequence and 64-row tile in the three dimensions of a grid, so that the
-// tiles of one length run together. The third dimension holds 65535; the tiles of longer sequences (4 194 240 tokens) are
-// folded into the first (not always: a block's two divisions cost 0.3 us a kernel, 3 % of a short call).
+// The fp32 attention kernels take one block per head, sequence and 64-row tile, in the three dimensions of a grid, so that the
+// tiles of one length run together. The third holds 65535, so sequences of more than 4 194 240 tokens take further
+// launches: how many tiles the launch that starts with tile `first` takes, 0 or less when there are none left. (Folding
+// the tiles into one dimension cost each block two divisions, 3 % of a short call.)
 constexpr int ATT_TILE = 64;
-struct AttBlock {
-  int head, seq, tile;  // tile may lie past the last one where tiles are folded
-};
-inline dim3 att_grid(int B, int T, int NH) {
-  const unsigned tiles = ((unsigned)T + ATT_TILE - 1) / ATT_TILE, folds = (tiles + 65534u) / 65535u;
-  return dim3(NH * folds, B, (tiles + folds - 1) / folds);
-}
-__host__ __device__ inline AttBlock att_block(unsigned x, unsigned y, unsigned z, unsigned grid_x, unsigned NH) {
-  if (grid_x == NH) return {(int)x, (int)y, (int)z};
-  return {(int)(x % NH), (int)y, (int)(z * (grid_x / NH) + x / NH)};
+inline int att_launch_tiles(int T, int first) {
+  const int left = (int)(((unsigned)T + ATT_TILE - 1) / ATT_TILE) - first;
+  return left < 65535 ? left : 65535;
 }
 
 int embedding_forward(float *out, const int *tokens, const float *wte, const float *wpe, int B, int T, int C, int Vp,

@@ -289,6 +289,7 @@ gpt2l_step *gpt2_schedule_instructions(gpt2_model *m, const int *tokens, const i
     // two backward GEMMs
     OpSpec g = gemm_spec(GPT2L_OP_FORWARD, M, C, Vp, m->logits, nullptr, m->lnf, P + m->off_wte, nullptr, o, L);
     g.gemm.opts.deterministic = 0;
+    g.gemm.opts.cta_pair = 1;  // as the list will be planned: it holds more than GEMMs
     g.gemm.xent_vocab = V;
     g.gemm.xent_stats = reinterpret_cast<float *>(16);  // placeholder while the tiling is planned
     GemmOp probe;

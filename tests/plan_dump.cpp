@@ -2,8 +2,8 @@
 //   mode kind M K N split_k cta_pair deterministic aux gelu stats  ->  error pair bn splits kb_per_split tiles_n
 // With the argument "simt", the CUDA-core GEMM's plan instead:
 //   Mc Nc Kc max_parts  ->  tile rows, tile columns, parts, k per part
-// With "attention", the grid of the fp32 attention kernels and its blocks (of large ones the first and the last layer):
-//   B T NH  ->  grid x y z, then head, sequence and tile of each block
+// With "attention", the launches of the fp32 attention kernels:
+//   T  ->  64-row tiles of each launch
 #include <cstdio>
 #include <cstring>
 
@@ -20,17 +20,9 @@ static int simt() {
 }
 
 static int attention() {
-  int B, T, NH;
-  while (scanf("%d %d %d", &B, &T, &NH) == 3) {
-    const dim3 g = g2l::att_grid(B, T, NH);
-    printf("%u %u %u", g.x, g.y, g.z);
-    const bool all = (long long)g.x * g.y * g.z <= 4096;
-    for (unsigned z = 0; z < g.z; z += all ? 1 : (g.z > 1 && z == 0 ? g.z - 1 : g.z))
-      for (unsigned y = 0; y < g.y; ++y)
-        for (unsigned x = 0; x < g.x; ++x) {
-          const g2l::AttBlock k = g2l::att_block(x, y, z, g.x, NH);
-          printf(" %d %d %d", k.head, k.seq, k.tile);
-        }
+  int T;
+  while (scanf("%d", &T) == 1) {
+    for (int first = 0, n; (n = g2l::att_launch_tiles(T, first)) > 0; first += n) printf("%d ", n);
     printf("\n");
   }
   return 0;
