@@ -360,7 +360,7 @@ __device__ __noinline__ bool row_op_tile(const GemmOp *op, const Tile &tc, int w
     case OPK_XENT: ok = row_xent(op, tile, w8, lane, scratch, rs, p); break;
     case OPK_ROWDOT: row_rowdot(op, tile, wtid); break;
     case OPK_ADAMW: row_adamw(op, tile, wtid, p); break;
-    case OPK_TRANSPOSE: row_transpose(op, tile, w8, lane, scratch + w8 * 1024); break;
+    case OPK_TRANSPOSE: ok = row_transpose(op, tile, w8, lane, scratch + w8 * 1024, rs, p); break;
     case OPK_XENT_COMBINE: row_xent_combine(op, tile, w8, lane); break;
     case OPK_XENT_GRAD: row_xent_grad(op, tile, wtid); break;
     default: break;

@@ -270,6 +270,7 @@ __device__ __forceinline__ bool row_xent(const GemmOp *op, int tile, int w8, int
   const float L2E = 1.4426950408889634f;
   const int r0 = tile * op->rows_per_tile;
   const int r1 = min(M, r0 + op->rows_per_tile);
+  if (!rs_.sync(p, op->op_index, lane)) return false;  // `red` lives in a GEMM epilogue box: every warp has left the last tile
   for (int rowi = r0; rowi < r1; ++rowi) {
     float *row = a.out0 + (long long)rowi * Vp;
     float m = -INFINITY, s = 0.f;
@@ -344,7 +345,7 @@ __device__ __forceinline__ bool row_xent(const GemmOp *op, int tile, int w8, int
       }
     }
   }
-  // `red` lives in a GEMM epilogue box as well
+  // nor does anyone move on to a GEMM tile's boxes before every warp has read `red`
   return rs_.sync(p, op->op_index, lane);
 }
 
@@ -480,11 +481,15 @@ __device__ __forceinline__ void row_adamw(const GemmOp *op, int tile, int wtid, 
 }
 
 // ---- out[c][m] = in[m][c] for the tile's rows: 32 x 32 blocks through a padded shared-memory box per warp ---
-__device__ __forceinline__ void row_transpose(const GemmOp *op, int tile, int w8, int lane, float *box /* 32 x 32 */) {
+// The boxes are the GEMM epilogues' staging boxes, dealt out to the warps differently there: nobody may write one before every
+// warp has left the GEMM tile before this one, nor move on to the next while another warp is still in its box.
+__device__ __forceinline__ bool row_transpose(const GemmOp *op, int tile, int w8, int lane, float *box /* 32 x 32 */, RowSync &rs_,
+                                              const LaunchParams &p) {
   const RowArgs &a = op->ra;
   const int M = a.i0, C = a.i1;
   const int r0 = tile * op->rows_per_tile;
   const int nrb = op->rows_per_tile / 32, ncb = (C + 31) / 32;
+  if (!rs_.sync(p, op->op_index, lane)) return false;
   for (int blk = w8; blk < nrb * ncb; blk += NUM_WORKER_WARPS) {
     const int rb = blk / ncb, cb = blk % ncb;
     const int m0 = r0 + rb * 32, c0 = cb * 32;
@@ -504,6 +509,7 @@ __device__ __forceinline__ void row_transpose(const GemmOp *op, int tile, int w8
       if (c < C && m < M) a.out0[(long long)c * M + m] = box[lane * 32 + (r ^ lane)];
     }
   }
+  return rs_.sync(p, op->op_index, lane);
 }
 
 }  // namespace g2l

@@ -110,6 +110,26 @@ def test_whole_gemm_set_in_one_launch(gpu):
     sched.close()
 
 
+def test_transposed_copies_survive_the_next_tile(gpu):
+    """A wide weight gradient reads a transposed copy that the list makes first, in the boxes that the next GEMM tile's
+    epilogue stages its stores in. New activations for every run, so that a block of an older copy would be seen."""
+    B, S, K, N = 8, 256, 768, 8192
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    x, w, dy = (torch.randn(s, device="cuda", generator=gen) for s in ((B * S, K), (K, K), (B * S, N)))
+    y, dw = torch.empty((B * S, K), device="cuda"), torch.empty((K, N), device="cuda")
+    o = gpu.make_opts(mode=0)
+    sched = gpu.Schedule([gpu.make_op(gpu.OP_FORWARD, B, S, K, K, y, x, w, opts=o),
+                          gpu.make_op(gpu.OP_BACKWARD_WEIGHT, B, S, K, N, dw, x, dy, opts=o)])
+    torch.backends.cuda.matmul.allow_tf32 = False
+    for _ in range(100):
+        x.normal_(generator=gen)
+        assert sched.run() == 0
+        for got, want in ((y, x @ w), (dw, x.t() @ dy)):
+            assert float((got - want).abs().max() / want.abs().max()) <= 2e-3  # (TF32 operands; a wrong block is off by 0.3)
+    assert sched.status() == 0
+    sched.close()
+
+
 def test_unsatisfiable_dependency_times_out_cleanly(gpu):
     """Host-side fault injection: the consumer is told to wait for more arrivals than its
     producer will ever publish. The launch must end by itself with the timeout status, name the
