@@ -724,7 +724,9 @@ gpt2_linear_tcgen05_kernel(const __grid_constant__ GemmOp op0, const LaunchParam
         continue;
       } else if (op->xform) {
         if (helper) ok = xform_tile<X3, MEGA>(op, tc, ring_ptr, rg, ctrl, p, pos, x, lane);
-        else ok = epilogue_tile<false>(op, maps, tc, tc.m_tile, tcount, false, 1, 0, 2u, 2u, sbuf, sbuf + EPI_BUF_BYTES, tmem_base, ctrl, p, warp, lane);
+        // (a second box only in 3xTF32 lists, where the helper warp it belongs to never drains a tile: in TF32 lists that warp may be
+        // at its share of the next op's tile while this one is drained)
+        else ok = epilogue_tile<false>(op, maps, tc, tc.m_tile, tcount, false, 1, 0, 2u, 2u, sbuf, X3 ? sbuf + EPI_BUF_BYTES : sbuf, tmem_base, ctrl, p, warp, lane);
         if (!helper) pos.skip(tc.kb1 - tc.kb0, rg.stages);
         ++tcount;
       } else {

@@ -172,3 +172,32 @@ def test_wide_rows_equal_the_separate_launches(gpu, monkeypatch, n_embd):
     for lo, hi in zip(bounds, bounds[1:]):
         a, b = res[1][1][lo:hi], res[0][1][lo:hi]
         assert np.isfinite(a).all() and np.abs(a - b).max() <= 5e-4 * max(np.abs(b).max(), 1e-12), (lo, np.abs(a - b).max())
+
+
+def test_loss_gradient_inside_the_gemms_equals_the_separate_launches(gpu, monkeypatch):
+    """GPT2_XENT=fused in TF32: the lm_head's backward tiles take a CTA's transform warps, the tiles of the ops around them do
+    not, so the two kinds of tile share staging boxes. One layer, several steps without the update, each against the launches
+    (the same TF32 products summed in another order: far below the 1e-2 that a foreign box of 32 x 32 would exceed)."""
+    monkeypatch.setenv("GPT2_XENT", "fused")
+    vocab, C, B, T = 1024, 768, 4, 128
+    params = gpt2_ref.to_flat(gpt2_ref.init_params(vocab, T, 1, C // 64, C), 1, vocab)
+    rng = np.random.default_rng(8)
+    tok, tgt = (torch.from_numpy(rng.integers(0, vocab, B * T).astype(np.int32)).cuda() for _ in range(2))
+    m = gpu.Model(vocab, vocab, 1, C // 64, C, T, B, T, mode=0)
+    m.set_params(params)
+    assert m.forward(tok, tgt) == 0 and m.backward() == 0
+    want, loss = np.empty_like(params), m.mean_loss()
+    m.get_grads(want)
+    bounds = m.offsets() + [m.num_params]
+    st = gpu.Step(m, tok, tgt, with_update=False)
+    for _ in range(10):
+        assert st.run() == 0
+        torch.cuda.synchronize()
+        got = np.empty_like(params)
+        m.get_grads(got)
+        assert abs(m.mean_loss() - loss) <= 1e-4
+        for lo, hi in zip(bounds, bounds[1:]):
+            assert np.abs(got[lo:hi] - want[lo:hi]).max() <= 1e-2 * max(np.abs(want[lo:hi]).max(), 1e-12), lo
+    assert st.status() == 0
+    st.close()
+    m.close()
